@@ -27,6 +27,7 @@
 // bit-reproducible); a finishing pass per slab converts to float and applies
 // the MLEM update f <- f * Ht / sens.
 #include "exact_device.cuh"
+#include "gather_device.cuh"
 #include "internal.h"
 
 #include <algorithm>
@@ -221,18 +222,6 @@ constexpr int kGatherTileX = 4;
 // SLOTS: voxels per lane and chunk (chunks of 32 * SLOTS slices; 8 unless the
 // volume is shorter)
 
-struct GatherConst {
-    float eu, ou;  // detector column of a point (a, b) of the view frame: a / (b + Rf) * eu + ou
-    float ez, oz;  // detector row of height z at depth d (t = d - Rf):      z / d * ez + oz
-    int vec4;      // X % 4 == 0 and the volume, sensitivity 16-byte aligned: float4 epilogue
-};
-
-// MLEM update of one voxel, as update_kernel computes it
-__device__ __forceinline__ float gather_update(float f, float ht, float sens)
-{
-    return (sens != 0.0f) ? __fdiv_rn(__fmul_rn(f, ht), sens) : 0.0f;
-}
-
 // The CTA's epilogue for one chunk of planes, coalesced along x.  Warp
 // w = xl + kGatherTileX * yl (column i0 + xl, j0 + yl) has left its sum for
 // entry e in stage[w * NE + e]; entry e belongs to plane zplane(e), or to none
@@ -273,75 +262,6 @@ __device__ __forceinline__ void gather_tile_epilogue(const ExactGeom& G, bool ve
             vol[v] = (EPI == 1) ? gather_update(vol[v], h, sens[v]) : h;
         }
     }
-}
-
-// A warp's column seen from one view: detector columns u_lo..u_hi and, for the
-// first two (sl = 0, 1), the column's piece [A, B] of their rays, the row
-// coefficients ca = ez / (A + Rf), cb = ez / (B + Rf) and the per-slot steps
-// pa = 32 vz ca, pb = 32 vz cb of the row bounds.  flags: bit sl = the rays of
-// u_lo + sl cross the column (A < B); bit 2 + sl = no voxel of the column has
-// a second candidate row there; bit 4 + sl = the piece lies behind the source
-// (every row is a candidate).
-struct GatherView {
-    float4 ab[2];  // {A, B, pa, pb}
-    float2 c[2];   // {ca, cb}
-    int u_lo, u_hi;
-    unsigned flags;
-    unsigned view;  // the view's index (fills the struct's 16-byte alignment)
-};
-
-// Column (i, j) of the volume, [Xa, Xb] x [Ya, Yb], seen from one view (see
-// GatherView); margin = the candidate rows' total widening (0.004 row).
-__device__ __forceinline__ GatherView gather_view(const ExactGeom& G, const GatherConst& C,
-                                                  const float4* __restrict__ txy, const int2* __restrict__ kxy,
-                                                  const float2* __restrict__ cs, unsigned view, int i, int j, float Xa,
-                                                  float Xb, float Ya, float Yb, float margin, float dz32)
-{
-    const float2 CS = __ldg(cs + view);
-    float umin = 3.0e38f, umax = -3.0e38f;
-    bool behind = false;
-#pragma unroll
-    for (int c4 = 0; c4 < 4; ++c4) {
-        const float X = (c4 & 1) ? Xb : Xa, Y = (c4 & 2) ? Yb : Ya;
-        const float a = X * CS.x - Y * CS.y, b = X * CS.y + Y * CS.x;
-        const float d = b + G.Rf;
-        behind |= !(d > 1e-3f * G.Rf);
-        const float uf = a / d * C.eu + C.ou;
-        umin = fminf(umin, uf);
-        umax = fmaxf(umax, uf);
-    }
-    GatherView V;
-    V.flags = 0u;
-    V.view = view;
-    if (behind) {  // not for a volume in front of the source; stays exact anyway
-        V.u_lo = 0;
-        V.u_hi = G.Nu - 1;
-    } else {
-        V.u_lo = min(max(0, __float2int_ru(umin - 0.01f)), G.Nu);
-        V.u_hi = min(G.Nu - 1, __float2int_rd(umax + 0.01f));
-    }
-#pragma unroll
-    for (int sl = 0; sl < 2; ++sl) {
-        const int u = min(V.u_lo + sl, G.Nu - 1);
-        const float4 T = __ldg(txy + (size_t)view * G.Nu + u);
-        const int2 K = __ldg(kxy + (size_t)view * G.Nu + u);
-        const float xa = plane_t(i, T.x, T.y, K.x), xb = plane_t(i + 1, T.x, T.y, K.x);
-        const float ya = plane_t(j, T.z, T.w, K.y), yb = plane_t(j + 1, T.z, T.w, K.y);
-        const float A = fmaxf(fminf(xa, xb), fminf(ya, yb));
-        const float B = fminf(fmaxf(xa, xb), fmaxf(ya, yb));
-        const float ca = C.ez / (A + G.Rf), cb = C.ez / (B + G.Rf);
-        V.ab[sl] = make_float4(A, B, dz32 * ca, dz32 * cb);
-        V.c[sl] = make_float2(ca, cb);
-        if (A < B) V.flags |= 1u << sl;
-        // a voxel's candidate interval [f0, f1] (row units) has a length
-        // convex in its height, largest at the column's bottom or top voxel
-        const float zb = G.P0[2], zt = G.P0[2] + (float)G.Z * G.vox[2];
-        const float len_b = fmaxf((zb + G.vox[2]) * ca, (zb + G.vox[2]) * cb) - fminf(zb * ca, zb * cb);
-        const float len_t = fmaxf(zt * ca, zt * cb) - fminf((zt - G.vox[2]) * ca, (zt - G.vox[2]) * cb);
-        if (fmaxf(len_b, len_t) + margin < 0.99f) V.flags |= 1u << (2 + sl);
-        if (!(A + G.Rf > 1e-3f * G.Rf)) V.flags |= 1u << (4 + sl);
-    }
-    return V;
 }
 
 template <int EPI, class ST, int SLOTS>
@@ -785,7 +705,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, 3) bp_gather_pairs_kernel(
     const float dz32 = 32.0f * G.vox[2];
     const int Zh = G.Z / 2;
     const unsigned top = (unsigned)G.Nv - 1u;
-    const unsigned Nh = (unsigned)G.Nv / 2u, Np = Nh + 1u;  // pairs per detector column
+    const unsigned Nh = (unsigned)G.Nv / 2u, Np = pair_entries(G.Nv);  // entries per detector column
     for (int k0 = 0; k0 < Zh; k0 += 32 * PS) {
         const float fk0 = (float)(k0 + lane);
         const float zl0 = fmaf(fk0, G.vox[2], G.P0[2]), zh0 = zl0 + G.vox[2];
@@ -955,6 +875,8 @@ __global__ void __launch_bounds__(kGatherWarps * 32, 3) bp_gather_pairs_kernel(
 }
 
 
+// The quarter-turn gather without stages, for the geometries that the staged one
+// (gather_staged.cu) does not take.
 // The pair gather over a quarter set of a plan's views (base views m0 .. m0 +
 // mc - 1 and their turns by one, two and three quarters; all views for m0 = 0,
 // mc = N/4) where views a quarter turn apart are exact rotations of each other (Plan::quarter, tables from
@@ -1008,7 +930,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, PS <= 2 ? 3 : 2) bp_gather_
     const float dz32 = 32.0f * G.vox[2];
     const int Zh = G.Z / 2;
     const unsigned top = (unsigned)G.Nv - 1u;
-    const unsigned Nh = (unsigned)G.Nv / 2u, Np = Nh + 1u;  // pairs per detector column
+    const unsigned Nh = (unsigned)G.Nv / 2u, Np = pair_entries(G.Nv);  // entries per detector column
     for (int k0 = 0; k0 < Zh; k0 += 32 * PS) {
         const float fk0 = (float)(k0 + lane);
         const float zl0 = fmaf(fk0, G.vox[2], G.P0[2]), zh0 = zl0 + G.vox[2];
@@ -1218,24 +1140,29 @@ __global__ void __launch_bounds__(256) to_pairs_kernel(const T* __restrict__ in,
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int u = u0 + threadIdx.y + 8 * q, p = p0 + threadIdx.x;
-        if (u >= Nu || p >= Np) continue;
+        if (u >= Nu || p >= pair_entries(Nv)) continue;
+        T* const o = out + (((size_t)blockIdx.z * Nu + u) * pair_entries(Nv) + p) * 2;
+        if (p >= Np) {  // padding
+            store_pair<T>(o, 0.0f, 0.0f);
+            continue;
+        }
         const float wa = wq ? __ldg(wq + (size_t)u * Nv + p) : 1.0f;
         const float wb = wq ? __ldg(wq + (size_t)u * Nv + (Nv - 1 - p)) : 1.0f;
-        store_pair<T>(out + (((size_t)blockIdx.z * Nu + u) * Np + p) * 2, lo[threadIdx.x][threadIdx.y + 8 * q] * wa,
-                      hi[threadIdx.x][threadIdx.y + 8 * q] * wb);
+        store_pair<T>(o, lo[threadIdx.x][threadIdx.y + 8 * q] * wa, hi[threadIdx.x][threadIdx.y + 8 * q] * wb);
     }
 }
 
 // wq (detector columns [u][v]) into mirrored row pairs.
 __global__ void wq_pairs_kernel(const float* __restrict__ wq, int Nu, int Nv, float* __restrict__ out)
 {
-    const int Np = Nv / 2 + 1;
+    const int Np = pair_entries(Nv);
     const size_t n = (size_t)Nu * Np;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
         const size_t u = q / Np;
         const int p = (int)(q % Np);
-        out[2 * q] = wq[u * Nv + p];
-        out[2 * q + 1] = wq[u * Nv + (Nv - 1 - p)];
+        const bool in = p <= Nv / 2;  // the padding entries hold 0
+        out[2 * q] = in ? wq[u * Nv + p] : 0.0f;
+        out[2 * q + 1] = in ? wq[u * Nv + (Nv - 1 - p)] : 0.0f;
     }
 }
 
@@ -1996,7 +1923,7 @@ recon_status_t exact_tune_bp(Plan& P)
 // arrays, within the 227 KB a block may use.
 int exact_bp_gather_max_rows() { return 12288; }
 
-static exact::GatherConst gather_const(const Plan& P, const float* vol, const float* sens)
+exact::GatherConst gather_const(const Plan& P, const float* vol, const float* sens)
 {
     const ExactGeom& E = P.eg;
     exact::GatherConst C;
@@ -2121,6 +2048,10 @@ static recon_status_t launch_gather(Plan& P, const ST* vals, size_t view_stride,
     if (P.z_mirror) {
         if (quarter_gather_serves<kQuarterSlots>(P, first, count)) {
             const unsigned q = P.nviews / 4;
+            bool served = false;
+            const recon_status_t st = staged_quarter_gather<EPI, ST>(P, vals, view_stride, vol, sens, s, npairs, false,
+                                                                     0u, q, &served);
+            if (st != RECON_OK || served) return st;
             switch (gather_quarter_slots(P.eg.Z)) {
                 case 1: return launch_gather_quarter<EPI, ST, 1>(P, vals, view_stride, vol, sens, s, npairs, 0u, q);
                 case 2: return launch_gather_quarter<EPI, ST, 2>(P, vals, view_stride, vol, sens, s, npairs, 0u, q);
@@ -2162,6 +2093,10 @@ recon_status_t exact_bp_quarters(Plan& P, unsigned first, unsigned count, float*
     auto run = [&](auto tag) -> recon_status_t {
         using ST = decltype(tag);
         const ST* vals = static_cast<const ST*>(P.d_ratio);
+        bool served = false;
+        const recon_status_t st = staged_quarter_gather<0, ST>(P, vals, qv, vol, nullptr, s, nullptr, true, first, count,
+                                                               &served);
+        if (st != RECON_OK || served) return st;
         switch (gather_quarter_slots(P.eg.Z)) {
             case 1: return launch_gather_quarter<0, ST, 1, true>(P, vals, qv, vol, nullptr, s, nullptr, first, count);
             case 2: return launch_gather_quarter<0, ST, 2, true>(P, vals, qv, vol, nullptr, s, nullptr, first, count);
@@ -2238,7 +2173,7 @@ bool exact_pairs_suit(const Plan& P)
 recon_status_t build_wq_pairs(Plan& P)
 {
     if (P.d_wq_pairs) return RECON_OK;
-    const size_t n = (size_t)P.eg.Nu * (P.eg.Nv / 2 + 1);
+    const size_t n = (size_t)P.eg.Nu * pair_entries(P.eg.Nv);
     RB_CHECK(P.alloc(&P.d_wq_pairs, 2 * n, "ray weights (mirrored row pairs)"));
     exact::wq_pairs_kernel<<<(unsigned)std::min<size_t>((n + 255) / 256, 148 * 8), 256>>>(P.d_wq, P.eg.Nu, P.eg.Nv,
                                                                                          P.d_wq_pairs);
@@ -2273,7 +2208,7 @@ recon_status_t exact_bp(Plan& P, const void* sino, bool sino_is_rw, bool bf16, u
         RB_CHECK(ensure_column_scratch(P, count));
         if (P.col_pairs) {
             const ExactGeom& E = P.eg;
-            exact::to_pairs_kernel<float><<<dim3((E.Nu + 31) / 32, (E.Nv / 2 + 1 + 31) / 32, count), dim3(32, 8), 0, s>>>(
+            exact::to_pairs_kernel<float><<<dim3((E.Nu + 31) / 32, (pair_entries(E.Nv) + 31) / 32, count), dim3(32, 8), 0, s>>>(
                 (const float*)sino, P.d_wq, E.Nu, E.Nv, P.d_colsino);
             RB_CUDA(cudaGetLastError());
         } else {

@@ -468,7 +468,7 @@ __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __
             if (MIRROR) out[base + (size_t)u * G.Nv + (G.Nv - 1 - v)] += sum.y;
         } else if constexpr (LAYOUT == kLayoutPairs) {
             static_assert(MIRROR, "mirrored row pairs come from the mirror-paired walk");
-            const int Np = G.Nv / 2 + 1;
+            const int Np = pair_entries(G.Nv);
             OT* const o = out + ((size_t)(view - view0) * G.Nu + u) * Np * 2;
             const float a = value(v, sum.x), b = value(G.Nv - 1 - v, sum.y);
             store_pair<OT>(o + 2 * v, a, b);
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(256) column_finish_pairs_kernel(ExactGeom G, c
                                                                   const GT* __restrict__ g, OT* __restrict__ out)
 {
     __shared__ float lo[32][33], hi[32][33];
-    const int Np = G.Nv / 2 + 1;
+    const int Np = G.Nv / 2 + 1;  // pairs; a column holds pair_entries(Nv) entries
     const int u0 = blockIdx.x * 32, p0 = blockIdx.y * 32;
     const size_t base = (size_t)blockIdx.z * G.Nu * G.Nv;
     if (MODE != 0) {
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(256) column_finish_pairs_kernel(ExactGeom G, c
         };
         const float a = value(p, MODE ? lo[threadIdx.x][threadIdx.y + 8 * q] : 0.0f);
         const float b = value(G.Nv - 1 - p, MODE ? hi[threadIdx.x][threadIdx.y + 8 * q] : 0.0f);
-        store_pair<OT>(out + (((size_t)blockIdx.z * G.Nu + u) * Np + p) * 2, a, b);
+        store_pair<OT>(out + (((size_t)blockIdx.z * G.Nu + u) * pair_entries(G.Nv) + p) * 2, a, b);
     }
 }
 

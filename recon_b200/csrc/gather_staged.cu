@@ -1,0 +1,647 @@
+// gather_staged.cu -- the EXACT gather back projector with its values staged in
+// shared memory by TMA.
+//
+// The gathers of exact.cu read each candidate row's value from L2 where they use
+// it, and a warp that owns a voxel column in registers leaves few warps to cover
+// that latency.  Here a CTA owns a tile of columns (one warp each) and one more
+// warp streams in what the tile reads: for every view the few detector columns
+// that the tile's shadow covers, cropped to the rows that its slices can meet
+// (one TMA box per view, completion on an mbarrier).  The column warps then find
+// every value in shared memory at 32-bit addresses.
+//
+// Measured (256^3, 360 views, 512^2; one B200): 1.56 ms against
+// bp_gather_quarter_kernel's 2.41 ms; 512^3, 720 views, 1024 x 768, BF16 ratio:
+// 22.8 against 40.2 ms.  Bound by shared-memory reads (about 80 % of their
+// wavefront peak: 52 wavefronts for the 1024 products of one detector column) with
+// 0.94e9 warp instructions (1.56e9).  What brought it there: loading the columns one
+// by one with untiled bulk copies 3.46 ms (28 copies a view, the loading warp the
+// limit), TMA boxes 2.10, two or four views to a stage instead of one 1.75, packed
+// multiply-adds without a predicate 1.56.  Reading the zero entry of a region in place
+// of the predicate cost bank conflicts (2.05).
+#include "exact_device.cuh"
+#include "gather_device.cuh"
+#include "internal.h"
+
+#include <cudaTypedefs.h>
+
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+
+namespace rb {
+namespace exact {
+
+// What a stage holds and how columns meet the detector, from the host (staged_shape).
+struct StagedShape {
+    int rows;     // staged entries per detector column (multiple of 4): the box's width
+    int cols;     // staged detector columns per view: the box's height
+    int stages;   // stages in flight
+    int wide;     // most detector columns one voxel column meets in a view: 1, 2, 4 or 8
+};
+
+// One detector column of one view as a voxel column sees it: the piece [A, B] of
+// its rays, row coefficients ca = ez / (A + Rf), cb = ez / (B + Rf), their steps
+// per slot (32 voxels) pa, pb, and the detector column u; one = no voxel of the
+// column has a second candidate row there.
+struct StagedItem {
+    float A, B, pa, pb, ca, cb;
+    int u, one;
+};
+
+// ---- bulk copies and their barriers --------------------------------------------------------
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(bar),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity)
+{
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity), "r"(1000000u)  // the warp may sleep up to 1 ms (ns) in one try
+        : "memory");
+    return done != 0u;
+}
+// Waits until the barrier's phase of this parity is complete; gives up after about
+// two seconds (false), which no run that works comes near.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity)
+{
+    if (mbar_try(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (!mbar_try(bar, parity))
+        if (clock64() - t0 > 4000000000ll) return false;
+    return true;
+}
+// The box at entry x (a multiple of four) of table row y into dst (128-byte aligned).
+__device__ __forceinline__ void tile_load(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            dst),
+        "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+
+// a += L * x in both halves: one packed instruction, each half rounded as fmaf.
+__device__ __forceinline__ void fma_pair(float2& a, float L, float2 x)
+{
+    unsigned long long acc = *reinterpret_cast<unsigned long long*>(&a);
+    const unsigned long long v = *reinterpret_cast<const unsigned long long*>(&x);
+    asm("{\n\t.reg .b64 l;\n\tmov.b64 l, {%1, %1};\n\tfma.rn.f32x2 %0, l, %2, %0;\n\t}" : "+l"(acc) : "f"(L), "l"(v));
+    a = *reinterpret_cast<float2*>(&acc);
+}
+
+// ---- the quarter-turn gather ----------------------------------------------------------------
+
+// bp_gather_quarter_kernel's sums (see there: one warp per base column of the
+// quadrant x, y < X/2, every length found at view m serving the voxel pair in the
+// four columns of its orbit at views m + rQ), in the same order, so the same bits.
+// A CTA owns TX x TY base columns (kWarps warps) and a loading warp; a stage holds
+// the four views' values of one base view, [r][detector column][row pair].
+constexpr int kStagedTX = 4, kStagedTY = 4;
+constexpr int kStagedWarps = kStagedTX * kStagedTY;
+constexpr int kStagedThreads = (kStagedWarps + 1) * 32;
+constexpr int kStageBytes = 98304;  // a stage: two or four base views of four regions of 12 or 6 KiB
+
+// Reads of shared memory at 32-bit addresses: a pair as stored (widen_lo / widen_hi
+// give its values), a row's z planes.
+__device__ __forceinline__ float2 lds_pair(unsigned a, float)
+{
+    float2 p;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(p.x), "=f"(p.y) : "r"(a));
+    return p;
+}
+__device__ __forceinline__ unsigned lds_pair(unsigned a, __nv_bfloat16)
+{
+    unsigned p;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(p) : "r"(a));
+    return p;
+}
+__device__ __forceinline__ float4 lds_planes(unsigned a)
+{
+    float4 p;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(a));
+    return p;
+}
+
+// Sum of |a| d / ... : the rows (relative to row 0) that heights [zb, zt] can be
+// seen at from depths [dmin, dmax], widened by one row.
+__device__ __forceinline__ void staged_rows(const GatherConst& C, float zb, float zt, float dmin, float dmax,
+                                            float& lo, float& hi)
+{
+    const float b0 = zb / dmin * C.ez, b1 = zb / dmax * C.ez, t0 = zt / dmin * C.ez, t1 = zt / dmax * C.ez;
+    lo = fminf(b0, b1) + C.oz - 1.0f;
+    hi = fmaxf(t0, t1) + C.oz + 1.0f;
+}
+
+// The first detector column that the rectangle [Xa, Xb] x [Ya, Yb] shadows at a view;
+// the columns that staged_item gives a voxel column inside it start there or later.
+__device__ __forceinline__ int staged_first_column(const ExactGeom& G, const GatherConst& C, const float2 CS, float Xa,
+                                                   float Xb, float Ya, float Yb)
+{
+    float umin = 3.0e38f;
+#pragma unroll
+    for (int c4 = 0; c4 < 4; ++c4) {
+        const float X = (c4 & 1) ? Xb : Xa, Y = (c4 & 2) ? Yb : Ya;
+        const float a = X * CS.x - Y * CS.y, b = X * CS.y + Y * CS.x;
+        umin = fminf(umin, __fdividef(a, b + G.Rf) * C.eu + C.ou);
+    }
+    return min(max(0, __float2int_ru(umin - 0.02f)), G.Nu - 1);
+}
+
+// Voxel column (i, j)'s item for detector column number sl of its range at a view;
+// valid when it returns true.
+__device__ __forceinline__ bool staged_item(const ExactGeom& G, const GatherConst& C, const float4* __restrict__ txy,
+                                            const int2* __restrict__ kxy, const float2 CS, unsigned view, int sl, int i,
+                                            int j, float Xa, float Xb, float Ya, float Yb, float margin, float dz32,
+                                            StagedItem& it)
+{
+    float umin = 3.0e38f, umax = -3.0e38f;
+#pragma unroll
+    for (int c4 = 0; c4 < 4; ++c4) {
+        const float X = (c4 & 1) ? Xb : Xa, Y = (c4 & 2) ? Yb : Ya;
+        const float a = X * CS.x - Y * CS.y, b = X * CS.y + Y * CS.x;
+        const float uf = __fdividef(a, b + G.Rf) * C.eu + C.ou;
+        umin = fminf(umin, uf);
+        umax = fmaxf(umax, uf);
+    }
+    const int u_lo = min(max(0, __float2int_ru(umin - 0.01f)), G.Nu);
+    const int u_hi = min(G.Nu - 1, __float2int_rd(umax + 0.01f));
+    it.u = u_lo + sl;
+    if (it.u > u_hi) return false;
+    const float4 T = __ldg(txy + (size_t)view * G.Nu + it.u);
+    const int2 K = __ldg(kxy + (size_t)view * G.Nu + it.u);
+    const float xa = plane_t(i, T.x, T.y, K.x), xb = plane_t(i + 1, T.x, T.y, K.x);
+    const float ya = plane_t(j, T.z, T.w, K.y), yb = plane_t(j + 1, T.z, T.w, K.y);
+    it.A = fmaxf(fminf(xa, xb), fminf(ya, yb));
+    it.B = fminf(fmaxf(xa, xb), fmaxf(ya, yb));
+    if (!(it.A < it.B)) return false;
+    it.ca = __fdividef(C.ez, it.A + G.Rf);
+    it.cb = __fdividef(C.ez, it.B + G.Rf);
+    it.pa = dz32 * it.ca;
+    it.pb = dz32 * it.cb;
+    // a voxel's candidate interval has a length convex in its height, largest at
+    // the column's bottom or top voxel
+    const float zb = G.P0[2], zt = G.P0[2] + (float)G.Z * G.vox[2];
+    const float len_b = fmaxf((zb + G.vox[2]) * it.ca, (zb + G.vox[2]) * it.cb) - fminf(zb * it.ca, zb * it.cb);
+    const float len_t = fmaxf(zt * it.ca, zt * it.cb) - fminf((zt - G.vox[2]) * it.ca, (zt - G.vox[2]) * it.cb);
+    it.one = (fmaxf(len_b, len_t) + margin < 0.99f) ? 1 : 0;
+    return true;
+}
+
+template <int EPI, class ST, int PS, int RB, bool SET>
+__global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
+    ExactGeom G, GatherConst C, StagedShape S, const float4* __restrict__ txy, const int2* __restrict__ kxy,
+    const float2* __restrict__ cs, const ZParam* __restrict__ zp, unsigned nview, unsigned m0, unsigned mc,
+    const __grid_constant__ CUtensorMap vals, unsigned view_rows, float* __restrict__ vol,
+    const float* __restrict__ sens, unsigned long long* __restrict__ npairs)
+{
+    constexpr unsigned kPair = 2 * sizeof(ST);  // bytes of a pair
+    constexpr int NE = 8 * PS * 32;  // epilogue entries per warp
+    constexpr int VB = kStageBytes / (4 * RB);  // base views per stage
+    constexpr int kMaxStages = 4;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ unsigned long long full[kMaxStages], empty[kMaxStages];
+    __shared__ int stage_u[kMaxStages * VB], first_u[32];
+    __shared__ StagedItem items[kStagedWarps][32];
+    unsigned char* const smem0 = smem + ((128u - (smem_addr(smem) & 127u)) & 127u);
+    float4* const szq = reinterpret_cast<float4*>(smem0);  // z planes of the staged rows, as in bp_gather_kernel
+    unsigned char* const stage0 = smem0 + (((size_t)S.rows * sizeof(float4) + 127) & ~(size_t)127);
+    float* const epi = reinterpret_cast<float*>(stage0);
+    const unsigned zq = smem_addr(szq), sq = smem_addr(stage0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int H = G.X / 2;
+    const int i0 = blockIdx.x * kStagedTX, j0 = blockIdx.y * kStagedTY;
+    const int i = i0 + warp % kStagedTX, j = j0 + (warp / kStagedTX) % kStagedTY;
+    const bool active = warp < kStagedWarps && i < H && j < H;
+    const unsigned nactive = (unsigned)(min(kStagedTX, H - i0) * min(kStagedTY, H - j0));
+    const unsigned Q = nview / 4u;
+    const unsigned nitem = SET ? 4u * mc : nview;
+    auto view_of = [&](unsigned it) { return SET ? m0 + it % mc + (it / mc) * Q : it; };
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S.stages; ++s) {
+            mbar_init(smem_addr(&full[s]), 1u);
+            mbar_init(smem_addr(&empty[s]), nactive);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const float Tx0 = G.P0[0] + i0 * G.vox[0], Tx1 = Tx0 + kStagedTX * G.vox[0];
+    const float Ty0 = G.P0[1] + j0 * G.vox[1], Ty1 = Ty0 + kStagedTY * G.vox[1];
+    const float Xa = G.P0[0] + i * G.vox[0], Xb = Xa + G.vox[0];
+    const float Ya = G.P0[1] + j * G.vox[1], Yb = Ya + G.vox[1];
+    const float rx = fmaxf(fabsf(Tx0), fabsf(Tx1)), ry = fmaxf(fabsf(Ty0), fabsf(Ty1));
+    const float rad = sqrtf(rx * rx + ry * ry) * 1.0001f;  // the tile's columns lie within it at every view
+    const float dz32 = 32.0f * G.vox[2];
+    const int Zh = G.Z / 2;
+    const int Nh = G.Nv / 2;
+    const unsigned nuse = (nitem + VB - 1) / VB;  // stage uses per chunk
+    unsigned base = 0;                            // and before this chunk
+    bool ok = true;
+    // A chunk's sums are taken with every product added, a row without a positive length
+    // as 0 * value.  Where a sum comes out not finite -- a value was not -- the chunk is
+    // taken again (exact) with only the products of positive lengths, which gives a value
+    // to the voxels that its ray crosses and to no others.
+    bool exact = EPI == 2;
+    for (int k0 = 0; k0 < Zh; base += nuse) {
+        // the rows that this chunk's lower voxels can meet, and their z planes
+        float flo, fhi;
+        staged_rows(C, G.P0[2] + (float)k0 * G.vox[2], G.P0[2] + (float)min(k0 + 32 * PS, Zh) * G.vox[2], G.Rf - rad,
+                    G.Rf + rad, flo, fhi);
+        const int p0 = min(max(0, (int)floorf(flo)), Nh) & ~3;
+        const int nrow = min(((min(Nh, max((int)ceilf(fhi), p0)) - p0 + 1) + 3) & ~3, S.rows);
+        __syncthreads();  // barriers set up; the last chunk's epilogue is done
+        for (int q = threadIdx.x; q < nrow; q += blockDim.x) {
+            const ZParam z = zp[min(p0 + q, G.Nv - 1)];
+            const float kc = (float)z.kc;
+            szq[q] = (z.S > 0.0f) ? make_float4(z.S, z.O, kc, kc - 1.0f) : make_float4(z.S, z.O, kc - 1.0f, kc);
+        }
+        if (k0 > 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        float2 acc[4][PS];  // {lower voxel, its mirror} in the four columns
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int s = 0; s < PS; ++s) acc[r][s] = make_float2(0.0f, 0.0f);
+        const int nslot = min(PS, max(0, (Zh - k0 - lane + 31) / 32));
+        if (warp == kStagedWarps) {
+            // the loading warp: VB items' detector columns into each stage, in turn
+            const unsigned bytes = 4u * (unsigned)(S.rows * S.cols) * kPair;
+            unsigned st = base % (unsigned)S.stages, ph = (base / (unsigned)S.stages) & 1u;
+            for (unsigned n = 0; n < nuse && ok; ++n) {
+                const unsigned i0 = n * VB, cnt = min((unsigned)VB, nitem - i0);
+                if (i0 % 32u == 0u) {  // 32 items' first detector columns, one per lane
+                    __syncwarp();
+                    if (i0 + lane < nitem)
+                        first_u[lane] = staged_first_column(G, C, __ldg(cs + view_of(i0 + lane)), Tx0, Tx1, Ty0, Ty1);
+                    __syncwarp();
+                }
+                ok = mbar_wait(smem_addr(&empty[st]), ph ^ 1u);
+                const unsigned bar = smem_addr(&full[st]);
+                if (ok && lane < VB) stage_u[st * VB + lane] = first_u[(i0 + lane) % 32u];
+                __syncwarp();
+                if (ok && lane == 0) {
+                    mbar_expect(bar, bytes * cnt);
+                    for (unsigned b = 0; b < cnt; ++b) {
+                        const int u = first_u[(i0 + b) % 32u];
+                        unsigned w = view_of(i0 + b);
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            tile_load(sq + st * kStageBytes + (b * 4 + r) * RB, &vals, p0, (int)(w * view_rows) + u, bar);
+                            w = (w + Q >= nview) ? w + Q - nview : w + Q;
+                        }
+                    }
+                }
+                if (!ok) {  // a warp does not answer: let the copies in flight land, then stop
+                    for (unsigned b = 1; b <= min(n, (unsigned)S.stages); ++b) {
+                        const unsigned use = base + n - b;
+                        mbar_wait(smem_addr(&full[use % (unsigned)S.stages]), (use / (unsigned)S.stages) & 1u);
+                    }
+                }
+                if (++st == (unsigned)S.stages) {
+                    st = 0;
+                    ph ^= 1u;
+                }
+            }
+        } else if (active) {
+            const float fk0 = (float)(k0 + lane);
+            const float zl0 = fmaf(fk0, G.vox[2], G.P0[2]), zh0 = zl0 + G.vox[2];
+            // rows relative to p0, with bp_gather_kernel's margins
+            const float oz_lo = C.oz - 0.002f - (float)p0, oz_hi = C.oz + 0.002f - (float)p0;
+            const unsigned last = (unsigned)nrow - 1u, colb = (unsigned)S.rows * kPair;
+            // row a of the staged rows: its length through lower voxel s of this lane, times
+            // its pairs in the four views (RB bytes apart from col)
+            auto add_row = [&](auto exact_tag, int s, float A, float B, unsigned a, unsigned col) {
+                const float4 zr = lds_planes(zq + a * 16u);
+                const float t = fk0 + (float)(32 * s);
+                const float lo = fmaf(t - zr.z, zr.x, zr.y), hi = fmaf(t - zr.w, zr.x, zr.y);
+                const float L = fminf(B, hi) - fmaxf(A, lo);
+                const unsigned x = col + a * kPair;
+                if constexpr (decltype(exact_tag)::value) {
+                    if (!(L > 0.0f)) return;
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const auto p = lds_pair(x + r * RB, ST());
+                        acc[r][s].x = (EPI == 2) ? acc[r][s].x + 1.0f : fmaf(L, widen_lo(p), acc[r][s].x);
+                        acc[r][s].y = (EPI == 2) ? acc[r][s].y + 1.0f : fmaf(L, widen_hi(p), acc[r][s].y);
+                    }
+                } else {
+                    const float Lp = fmaxf(L, 0.0f);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const auto p = lds_pair(x + r * RB, ST());
+                        fma_pair(acc[r][s], Lp, make_float2(widen_lo(p), widen_hi(p)));
+                    }
+                }
+            };
+            // one detector column, several candidate rows per voxel or exact sums: col = the
+            // first view's pairs of it
+            auto rows_general = [&](auto exact_tag, const StagedItem& I, unsigned col) {
+                const float P0a = fmaf(zl0, I.ca, oz_lo), P0b = fmaf(zl0, I.cb, oz_lo);
+                const float P1a = fmaf(zh0, I.ca, oz_hi), P1b = fmaf(zh0, I.cb, oz_hi);
+                unsigned a[PS];
+                int more = 0;  // further candidate rows of this lane's voxels, at most
+#pragma unroll
+                for (int s = 0; s < PS; ++s) {
+                    const float f0 = fminf(fmaf((float)s, I.pa, P0a), fmaf((float)s, I.pb, P0b));
+                    const float f1 = fmaxf(fmaf((float)s, I.pa, P1a), fmaf((float)s, I.pb, P1b));
+                    a[s] = min(__float2uint_ru(f0), last);
+                    more = max(more, min(__float2int_rd(f1), (int)last) - (int)a[s]);
+                }
+                more = __reduce_max_sync(0xffffffffu, more);
+                for (int n = 0; n <= more; ++n)
+#pragma unroll
+                    for (int s = 0; s < PS; ++s)
+                        if (n == 0 || a[s] + (unsigned)n <= last) add_row(exact_tag, s, I.A, I.B, a[s] + (unsigned)n, col);
+            };
+            const int wshift = __ffs(S.wide) - 1;
+            const int per = 32 / S.wide;  // views whose items a warp sets up at a time
+            unsigned st = base % (unsigned)S.stages, ph = (base / (unsigned)S.stages) & 1u;
+            for (unsigned vb = 0; vb < nitem; vb += per) {
+                const unsigned nb = min((unsigned)per, nitem - vb);
+                bool valid = false;
+                {
+                    const unsigned q = (unsigned)(lane / S.wide);
+                    StagedItem it;
+                    if (q < nb) {
+                        const unsigned m = view_of(vb + q);
+                        valid = staged_item(G, C, txy, kxy, __ldg(cs + m), m, lane % S.wide, i, j, Xa, Xb, Ya, Yb,
+                                            oz_hi - oz_lo, dz32, it);
+                        if (exact) it.one = 0;
+                        if (valid) items[warp][lane] = it;
+                    }
+                }
+                unsigned mask = __ballot_sync(0xffffffffu, valid);
+                __syncwarp();
+                for (unsigned q = 0; q < nb; q += VB) {
+                    // the stage's items: bits q wide .. (q + VB) wide - 1 of the mask
+                    unsigned mine = (S.wide * VB >= 32) ? mask : (mask >> (q * S.wide)) & ((1u << (S.wide * VB)) - 1u);
+                    if (ok) ok = mbar_wait(smem_addr(&full[st]), ph);
+                    for (; mine != 0u; mine &= mine - 1u) {
+                        const unsigned e = (unsigned)__ffs(mine) - 1u, b = e >> wshift;
+                        const StagedItem I = items[warp][q * S.wide + e];
+                        const unsigned col = sq + st * kStageBytes + b * (4 * RB) +
+                                             (unsigned)min(max(I.u - stage_u[st * VB + b], 0), S.cols - 1) * colb;
+                        if (I.one) {  // one candidate row per voxel, clamped to a staged row
+                            const float P0a = fmaf(zl0, I.ca, oz_lo);
+#pragma unroll
+                            for (int s = 0; s < PS; ++s)
+                                add_row(std::false_type{}, s, I.A, I.B,
+                                        min(__float2uint_ru(fmaf((float)s, I.pa, P0a)), last), col);
+                        } else if (exact) {
+                            rows_general(std::true_type{}, I, col);
+                        } else {
+                            rows_general(std::false_type{}, I, col);
+                        }
+                    }
+                    __syncwarp();  // the stage is read
+                    if (lane == 0) mbar_arrive(smem_addr(&empty[st]));
+                    if (++st == (unsigned)S.stages) {
+                        st = 0;
+                        ph ^= 1u;
+                    }
+                }
+                __syncwarp();  // the next batch rewrites the items
+            }
+            if (!ok) {  // a stage never came: the sums are not the answer
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int s = 0; s < PS; ++s) acc[r][s].x = acc[r][s].y = __int_as_float(0x7fffffff);
+            }
+        }
+        if (EPI != 2) {
+            bool bad = false;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int s = 0; s < PS; ++s) bad |= s < nslot && !(isfinite(acc[r][s].x) && isfinite(acc[r][s].y));
+            if (__syncthreads_or(bad && ok && !exact)) {
+                exact = true;
+                continue;
+            }
+            exact = false;
+        }
+        if (EPI == 2) {  // pair counts of the four columns
+            unsigned long long c = 0;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int s = 0; s < PS; ++s)
+                    if (s < nslot) c += (unsigned long long)acc[r][s].x + (unsigned long long)acc[r][s].y;
+            for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+            if (lane == 0 && c) atomicAdd(npairs, c);
+            k0 += 32 * PS;
+            continue;
+        }
+        // every stage is read (the barrier above): its memory takes the sums
+        if (warp < kStagedWarps) {
+            float* const o = epi + warp * NE;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int s = 0; s < PS; ++s) {
+                    o[((r * 2) * PS + s) * 32 + lane] = acc[r][s].x;
+                    o[((r * 2 + 1) * PS + s) * 32 + lane] = acc[r][s].y;
+                }
+        }
+        __syncthreads();
+        // one voxel per thread, the tile's columns fastest (x neighbours adjacent)
+        const size_t plane = (size_t)G.X * G.Y;
+        for (int q = threadIdx.x; q < kStagedWarps * NE; q += blockDim.x) {
+            const int w = q % kStagedWarps, e = q / kStagedWarps;
+            const int r = e / (2 * PS * 32), h = (e / (PS * 32)) & 1, k = k0 + e % (PS * 32);
+            // columns d_1 and d_3 run along x with the base column's y
+            const int wi = (r & 1) ? w / kStagedTX : w % kStagedTX, wj = (r & 1) ? w % kStagedTX : w / kStagedTX;
+            const int bi = i0 + wi, bj = j0 + wj;
+            if (bi >= H || bj >= H || k >= Zh) continue;
+            const int x = (r == 0) ? bi : (r == 1) ? bj : (r == 2) ? G.X - 1 - bi : G.X - 1 - bj;
+            const int y = (r == 0) ? bj : (r == 1) ? G.X - 1 - bi : (r == 2) ? G.X - 1 - bj : bi;
+            const int z = h ? G.Z - 1 - k : k;
+            const size_t v = (size_t)z * plane + (size_t)y * G.X + (size_t)x;
+            const float hv = epi[(wj * kStagedTX + wi) * NE + e];
+            vol[v] = (EPI == 1) ? gather_update(vol[v], hv, sens[v]) : hv;
+        }
+        k0 += 32 * PS;
+    }
+}
+
+}  // namespace exact
+
+// ---- host side -----------------------------------------------------------------------------
+
+// Detector columns whose rays can meet a rectangle of diagonal d mm anywhere in the
+// volume: its shadow is at most d * |Ry| / depth * sqrt(1 + tan^2) / du pitches wide.
+static int staged_span(const Plan& P, double d, double rad)
+{
+    const ExactGeom& E = P.eg;
+    const double dmin = (double)E.Rf - rad, tan = rad / dmin;
+    return (int)std::floor(d / dmin * std::sqrt(1.0 + tan * tan) * std::fabs((double)E.Ry / E.du) + 0.05) + 1;
+}
+
+// The stage layout for chunks of 32 * slots slices of the lower half, or false where the
+// staged gather does not serve and bp_gather_quarter_kernel does: a volume that comes
+// near the source (a piece could then lie behind it), a voxel column that meets more than
+// eight detector columns, a box of more than 256 a side or 12 KiB (a detector several
+// times finer than the voxels: its rows and columns then outgrow the two stages that a
+// block's shared memory holds).
+static bool staged_shape(const Plan& P, int slots, size_t value_bytes, exact::StagedShape* out, int* region,
+                         size_t* smem)
+{
+    const ExactGeom& E = P.eg;
+    const double vx = E.vox[0], vy = E.vox[1], vz = E.vox[2];
+    const double tx = exact::kStagedTX * vx, ty = exact::kStagedTY * vy;
+    const double rad = std::hypot(0.5 * E.X * vx + tx, 0.5 * E.Y * vy + ty) * 1.001;
+    if (!(rad < 0.9 * (double)E.Rf)) return false;
+    const double ez = (double)E.Ry / E.dv, oz = -((double)E.Dz + E.vd0) / E.dv;
+    exact::StagedShape S;
+    const int wide = staged_span(P, std::hypot(vx, vy), rad);
+    if (wide > 8) return false;
+    S.wide = wide <= 1 ? 1 : wide <= 2 ? 2 : wide <= 4 ? 4 : 8;
+    S.cols = staged_span(P, std::hypot(tx, ty), rad);
+    const int Zh = E.Z / 2, Nh = E.Nv / 2;
+    int rows = 0;
+    for (int k0 = 0; k0 < Zh; k0 += 32 * slots) {
+        const double zb = E.P0[2] + k0 * vz, zt = E.P0[2] + std::min(k0 + 32 * slots, Zh) * vz;
+        const double dn = E.Rf - rad, df = E.Rf + rad;
+        const double lo = std::min(zb / dn * ez, zb / df * ez) + oz - 2.0;
+        const double hi = std::max(zt / dn * ez, zt / df * ez) + oz + 2.0;
+        const int a = std::max(0, (int)std::floor(lo)) & ~3, b = std::min(Nh, (int)std::ceil(hi));
+        rows = std::max(rows, ((b - a + 1) + 3) / 4 * 4);
+    }
+    S.rows = std::max(rows, 4);
+    if (S.rows > 256 || S.cols > 256) return false;  // a box's sides
+    const size_t pair = 2 * value_bytes;
+    const size_t used = (size_t)S.cols * S.rows * pair;
+    if (used > 12288) return false;
+    *region = used <= 6144 ? 6144 : 12288;
+    const size_t planes = ((size_t)S.rows * sizeof(float4) + 127) / 128 * 128;
+    const size_t stage = exact::kStageBytes;
+    const size_t epilogue = sizeof(float) * exact::kStagedWarps * 8 * slots * 32;
+    const size_t fixed = sizeof(exact::StagedItem) * 32 * exact::kStagedWarps + 1024;  // static shared memory
+    const size_t room = 227 * 1024 - fixed - planes;
+    if (planes + fixed > 100 * 1024 || 2 * stage > room || epilogue > room) return false;
+    S.stages = (int)std::min<size_t>(4, room / stage);
+    *out = S;
+    *smem = 128 + planes + std::max((size_t)S.stages * stage, epilogue);  // 128: the base's alignment
+    return true;
+}
+
+// The driver's tensor map encoder, looked up once.
+static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
+{
+    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+    }();
+    return fn;
+}
+
+// Mirrored row pairs as a table of `table_rows` detector columns of pair_entries(Nv)
+// entries (an entry is moved as one 8- or 4-byte element), read in boxes of S.rows
+// entries x S.cols detector columns.
+static bool pair_map(const Plan& P, const exact::StagedShape& S, const void* vals, size_t pair_bytes, size_t table_rows,
+                     CUtensorMap* map)
+{
+    const auto encode = tensor_map_encoder();
+    if (!encode || reinterpret_cast<uintptr_t>(vals) % 16 != 0) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)pair_entries(P.eg.Nv), (cuuint64_t)table_rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)pair_entries(P.eg.Nv) * pair_bytes};
+    const cuuint32_t box[2] = {(cuuint32_t)S.rows, (cuuint32_t)S.cols}, step[2] = {1, 1};
+    return encode(map, pair_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_UINT32, 2,
+                  const_cast<void*>(vals), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int EPI, class ST, int PS, int RB, bool SET>
+static recon_status_t launch_staged(Plan& P, const exact::StagedShape& S, size_t smem, const CUtensorMap& map,
+                                    unsigned view_rows, float* vol, const float* sens, cudaStream_t s,
+                                    unsigned long long* npairs, unsigned m0, unsigned mc)
+{
+    const ExactGeom& E = P.eg;
+    auto kernel = exact::bp_staged_quarter_kernel<EPI, ST, PS, RB, SET>;
+    RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int H = E.X / 2;
+    const dim3 grid((H + exact::kStagedTX - 1) / exact::kStagedTX, (H + exact::kStagedTY - 1) / exact::kStagedTY);
+    kernel<<<grid, exact::kStagedThreads, smem, s>>>(E, gather_const(P, vol, sens), S, P.d_txy, P.d_kxy, P.d_cs, P.d_zp,
+                                                     P.nviews, m0, mc, map, view_rows, vol, sens, npairs);
+    RB_CUDA(cudaGetLastError());
+    return RECON_OK;
+}
+
+// Voxel pairs per lane: the lower half's height in as few chunks of at most 4 x 32
+// slices as possible, split evenly.
+static int staged_slots(int Z)
+{
+    const int half = Z / 2, chunks = (half + 127) / 128;
+    return std::min(4, std::max(1, (half + 32 * chunks - 1) / (32 * chunks)));
+}
+
+// The quarter-turn gather over base views m0 .. m0 + mc - 1 of each quarter (set), or
+// all views; *served = false (and nothing launched) where its stages do not fit.
+template <int EPI, class ST>
+recon_status_t staged_quarter_gather(Plan& P, const ST* vals, size_t view_stride, float* vol, const float* sens,
+                                     cudaStream_t s, unsigned long long* npairs, bool set, unsigned m0, unsigned mc,
+                                     bool* served)
+{
+    exact::StagedShape S;
+    size_t smem = 0;
+    int region = 0;
+    const int slots = staged_slots(P.eg.Z);
+    CUtensorMap map;
+    // view_stride 0: the same table for every view (the weights of the sensitivity)
+    const unsigned view_rows = view_stride ? (unsigned)P.eg.Nu : 0u;
+    const size_t table_rows = view_stride ? (size_t)P.eg.Nu * P.nviews : (size_t)P.eg.Nu;
+    *served = table_rows < 0x7fffffff && staged_shape(P, slots, sizeof(ST), &S, &region, &smem) &&
+              pair_map(P, S, vals, 2 * sizeof(ST), table_rows, &map);
+    if (!*served) return RECON_OK;
+    auto run = [&](auto ps) -> recon_status_t {
+        constexpr int PS = decltype(ps)::value;
+        auto go = [&](auto rb) -> recon_status_t {
+            constexpr int RB = decltype(rb)::value;
+            if constexpr (EPI == 0) {
+                if (set)
+                    return launch_staged<EPI, ST, PS, RB, true>(P, S, smem, map, view_rows, vol, sens, s, npairs, m0, mc);
+            }
+            return launch_staged<EPI, ST, PS, RB, false>(P, S, smem, map, view_rows, vol, sens, s, npairs, m0, mc);
+        };
+        return region == 6144 ? go(std::integral_constant<int, 6144>{}) : go(std::integral_constant<int, 12288>{});
+    };
+    switch (slots) {
+        case 1: return run(std::integral_constant<int, 1>{});
+        case 2: return run(std::integral_constant<int, 2>{});
+        case 3: return run(std::integral_constant<int, 3>{});
+        default: return run(std::integral_constant<int, 4>{});
+    }
+}
+
+#define RB_STAGED(EPI, ST)                                                                                          \
+    template recon_status_t staged_quarter_gather<EPI, ST>(Plan&, const ST*, size_t, float*, const float*,          \
+                                                           cudaStream_t, unsigned long long*, bool, unsigned, unsigned, \
+                                                           bool*);
+RB_STAGED(0, float)
+RB_STAGED(1, float)
+RB_STAGED(2, float)
+RB_STAGED(0, __nv_bfloat16)
+RB_STAGED(1, __nv_bfloat16)
+#undef RB_STAGED
+
+}  // namespace rb

@@ -81,7 +81,7 @@ struct DeviceBuf {
 // Layouts of a sinogram on the device: rows [view][v][u] (the reference's),
 // detector columns [view][u][v], or mirrored row pairs [view][u][p][2] holding
 // {row p, row Nv-1-p} for p = 0 .. Nv/2 (even Nv; entry Nv/2 repeats the last
-// pair swapped), which the mirror-paired gather reads with one load per pair.
+// pair swapped; columns padded to pair_entries), which the mirror-paired gather reads with one load per pair.
 enum : int { kLayoutRows = 0, kLayoutColumns = 1, kLayoutPairs = 2 };
 
 struct RayTiles {
@@ -193,12 +193,16 @@ recon_status_t Plan::alloc(T** p, size_t count, const char* what)
     return RECON_OK;
 }
 
+// Entries of one detector column in mirrored row pairs: Nv/2 + 1, padded to four so
+// that every column and every fourth entry start on 16 bytes (bulk copies).
+__host__ __device__ inline int pair_entries(int Nv) { return (Nv / 2 + 4) / 4 * 4; }
+
 // Elements one view of the gather's input occupies: Nu*Nv in detector columns,
-// Nu*(Nv/2 + 1)*2 in mirrored row pairs.
+// Nu*pair_entries(Nv)*2 in mirrored row pairs.
 inline size_t column_view_elems(const Plan& P)
 {
     if (!P.col_pairs) return P.npix;
-    return (size_t)P.geom.det.NumAxPixels * (P.geom.det.NumTAxPixels / 2 + 1) * 2;
+    return (size_t)P.geom.det.NumAxPixels * pair_entries((int)P.geom.det.NumTAxPixels) * 2;
 }
 
 // ---- entry points implemented in the .cu files --------------------------------
