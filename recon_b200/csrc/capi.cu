@@ -32,6 +32,7 @@ Plan::~Plan()
     cudaGetDevice(&cur);
     if (cur != device) cudaSetDevice(device);
     release_plan_textures(this);
+    if (vol_z_free) cudaEventDestroy(vol_z_free);
     for (void* p : allocations) cudaFree(p);
     if (cur >= 0 && cur != device) cudaSetDevice(cur);
 }
@@ -134,6 +135,7 @@ static void fill_geoms(Plan& P)
     C.Pd[0] = g.vox.XVoxSize;
     C.Pd[1] = g.vox.YVoxSize;
     C.Pd[2] = g.vox.ZVoxSize;
+    for (int k = 0; k < 3; ++k) C.inv_Pd[k] = 1.0f / C.Pd[k];
     C.Xs[0] = 0.0f;
     C.Xs[1] = -g.cal.Rf;
     C.Xs[2] = 0.0f;
@@ -329,6 +331,7 @@ recon_status_t recon_plan_create(const recon_geometry_t* geom, const recon_optio
             RB_CHECK(P->alloc(&P->d_fix, P->nvox, "fixed-point accumulator"));
             RB_CHECK(P->alloc(&P->d_ht, P->nvox, "Ht"));
             RB_CUDA(cudaMemset(P->d_fix, 0, P->nvox * sizeof(unsigned long long)));
+            RB_CHECK(compat_alloc_volume(*P));
             RB_CHECK(build_compat_tables(*P, 0));
         }
         // the set-up ran on the legacy stream; waiting for that stream alone (not the
@@ -439,11 +442,7 @@ recon_status_t recon_bp_views(recon_plan_t P, const float* d_sino, unsigned firs
     RB_CHECK(use_device(*P));
     cudaStream_t s = as_stream(stream);
     if (count == 0) return launch_fill(d_vol, 0.0f, P->nvox, s);
-    if (P->opt.arith == RECON_ARITH_COMPAT) {
-        for (unsigned n = 0; n < count; ++n)
-            RB_CHECK(compat_bp_view(*P, d_sino + (size_t)n * P->npix, first + n, false, 0.0f, d_vol, n > 0, s));
-        return RECON_OK;
-    }
+    if (P->opt.arith == RECON_ARITH_COMPAT) return compat_bp_views(*P, d_sino, first, count, d_vol, s);
     return exact_bp(*P, d_sino, false, false, first, count, false, false, d_vol, nullptr, nullptr, s);
 }
 

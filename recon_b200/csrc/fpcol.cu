@@ -509,19 +509,22 @@ constexpr auto fp_column_kernel_of()
 // through shared memory; the zero layers (z = -1 and z = Z) are set once when
 // the buffer is allocated and never written here.
 __global__ void __launch_bounds__(256) to_zfast_kernel(const float* __restrict__ in, float* __restrict__ out, int X,
-                                                       int Y, int Z)
+                                                       int Y, int Z, int pad)
 {
     __shared__ float tile[32][33];
-    const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 32, y = blockIdx.z;
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        const int x = x0 + threadIdx.x, z = z0 + r;
-        if (x < X && z < Z) tile[r][threadIdx.x] = in[((size_t)z * Y + y) * X + x];
-    }
-    __syncthreads();
-    const size_t Zp = (size_t)Z + 2;
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        const int z = z0 + threadIdx.x, x = x0 + r;
-        if (x < X && z < Z) out[((size_t)y * X + x) * Zp + z + 1] = tile[threadIdx.x][r];
+    const int tx = (X + 31) / 32, x0 = (int)(blockIdx.x % tx) * 32, z0 = (int)(blockIdx.x / tx) * 32;
+    const size_t Zp = (size_t)Z + 2 * pad;
+    for (int y = blockIdx.y; y < Y; y += gridDim.y) {
+        for (int r = threadIdx.y; r < 32; r += 8) {
+            const int x = x0 + threadIdx.x, z = z0 + r;
+            if (x < X && z < Z) tile[r][threadIdx.x] = in[((size_t)z * Y + y) * X + x];
+        }
+        __syncthreads();
+        for (int r = threadIdx.y; r < 32; r += 8) {
+            const int z = z0 + threadIdx.x, x = x0 + r;
+            if (x < X && z < Z) out[((size_t)y * X + x) * Zp + z + pad] = tile[threadIdx.x][r];
+        }
+        __syncthreads();
     }
 }
 
@@ -788,13 +791,17 @@ recon_status_t build_column_tiles(Plan& P, const std::vector<int4>& rect)
     return RECON_OK;
 }
 
-recon_status_t exact_to_zfast(const Plan& P, const float* vol, cudaStream_t s)
+recon_status_t launch_zfast(const float* vol, float* out, int X, int Y, int Z, int pad, cudaStream_t s)
 {
-    const ExactGeom& E = P.eg;
-    exact::to_zfast_kernel<<<dim3((E.X + 31) / 32, (E.Z + 31) / 32, E.Y), dim3(32, 8), 0, s>>>(vol, P.d_vol_z, E.X,
-                                                                                             E.Y, E.Z);
+    const dim3 grid((unsigned)((X + 31) / 32) * (unsigned)((Z + 31) / 32), std::min(Y, 65535));
+    exact::to_zfast_kernel<<<grid, dim3(32, 8), 0, s>>>(vol, out, X, Y, Z, pad);
     RB_CUDA(cudaGetLastError());
     return RECON_OK;
+}
+
+recon_status_t exact_to_zfast(const Plan& P, const float* vol, cudaStream_t s)
+{
+    return launch_zfast(vol, P.d_vol_z, P.eg.X, P.eg.Y, P.eg.Z, 1, s);
 }
 
 // Views [first, first + count) of table slots through the column kernel: the

@@ -39,6 +39,7 @@ struct CompatGeom {
     float R, Rf, Ry, Dx, Dz, M;
     float NumAxPixels_f, NumTAxPixels_f, AxPixDimMm, TAxPixDimMm;
     float Pi[3], Pf[3], Pd[3], Xs[3];
+    float inv_Pd[3];  // 1 / Pd: exact where Pd is a power of two, and used only there
     float RM[9];
     int dims[3];
     int Nu, Nv;
@@ -127,7 +128,9 @@ struct Plan {
     float* d_vol_t = nullptr;  // xy-transposed copy of the projected volume [z][x][y] (ray-walk forward projector)
     bool fp_column = false;    // forward projection by detector columns (fpcol.cu), else the ray walk
     float* d_vol_z = nullptr;  // z-fastest copy of the projected volume with a zero layer at each end:
-                               // voxel (x, y, z) at [(y*X + x)*(Z + 2) + z + 1] (column forward projector)
+                               // voxel (x, y, z) at [(y*X + x)*(Z + 2) + z + 1] (column forward projector);
+                               // COMPAT: without the layers, [(y*X + x)*Z + z]
+    cudaEvent_t vol_z_free = nullptr;  // COMPAT: the last use of d_vol_z
     // back projection: fixed-point accumulators of one z-slab, image layout
     // and xy-transposed, and the max |value| of the call's input (float bits)
     unsigned long long* d_bpacc = nullptr;
@@ -232,6 +235,10 @@ recon_status_t compat_fp(Plan& P, const float* vol, unsigned first, unsigned cou
 recon_status_t compat_bp_view(Plan& P, const float* img, unsigned view, bool scratch_slot,
                               float angle_scratch, float* out_or_accum, bool accumulate,
                               cudaStream_t s);
+recon_status_t compat_alloc_volume(Plan& P);
+recon_status_t compat_bp_views(Plan& P, const float* sino, unsigned first, unsigned count, float* out, cudaStream_t s);
+// vol[z][y][x] -> out[(y*X + x)*(Z + 2*pad) + z + pad] (fpcol.cu); the padding is not written
+recon_status_t launch_zfast(const float* vol, float* out, int X, int Y, int Z, int pad, cudaStream_t s);
 recon_status_t compat_mlem_iteration(Plan& P, const float* g, float* f, cudaStream_t s);
 recon_status_t compat_sensitivity(Plan& P, float* sens, cudaStream_t s);
 
