@@ -309,7 +309,20 @@ recon_status_t recon_plan_create(const recon_geometry_t* geom, const recon_optio
             } else {
                 RB_CHECK(P->alloc(&P->d_vol_t, P->nvox, "transposed volume"));
             }
-            if (!P->bp_gather || tuned) {  // the ray-driven back projector's slab accumulators
+            RB_CHECK(build_exact_tables(*P, 0));
+            RB_CHECK(exact_check_mirror(*P));
+            // both designs' inputs where they are measured, the chosen one's otherwise
+            const bool gather = P->bp_gather && !tuned;
+            if (gather || tuned) {
+                exact_use_gather(*P, true);
+                if (P->col_pairs) RB_CHECK(build_wq_pairs(*P));
+            }
+            if (!gather) exact_use_gather(*P, false);
+            if (P->bp_columns) {
+                RB_CHECK(build_view_maxima(*P));
+                RB_CHECK(P->alloc(&P->d_bpacc, bp_acc_words(*P), "back projection accumulator"));
+                RB_CHECK(P->alloc(&P->d_bpmax, 4, "back projection scale"));  // a FixScale
+            } else if (!gather) {  // the ray-driven back projector's slab accumulators
                 const size_t slab = (size_t)P->eg.X * P->eg.Y * bp_slab_depth(*P);
                 RB_CHECK(P->alloc(&P->d_bpacc, slab, "back projection accumulator"));
                 RB_CHECK(P->alloc(&P->d_bpacc_t, slab, "back projection accumulator (transposed)"));
@@ -317,20 +330,13 @@ recon_status_t recon_plan_create(const recon_geometry_t* geom, const recon_optio
                 RB_CUDA(cudaMemset(P->d_bpacc, 0, slab * sizeof(unsigned long long)));
                 RB_CUDA(cudaMemset(P->d_bpacc_t, 0, slab * sizeof(unsigned long long)));
             }
-            RB_CHECK(build_exact_tables(*P, 0));
-            RB_CHECK(exact_check_mirror(*P));
-            if (tuned) P->bp_gather = false;  // the culling builds the ray design's slab tiles too
             RB_CHECK(build_exact_culling(*P));
-            const bool pairs = exact_pairs_suit(*P) && (P->bp_gather || tuned);
-            if (pairs) RB_CHECK(build_wq_pairs(*P));
             if (tuned) RB_CHECK(exact_tune_bp(*P));
-            P->col_pairs = pairs && P->bp_gather;
             if (tuned && opt.fp_rows == 0) RB_CHECK(exact_tune_fp(*P));
         } else {
             RB_CHECK(P->alloc(&P->d_maxabs, nv1 + 1, "maxabs"));  // per view, scratch slot, all views
             RB_CHECK(P->alloc(&P->d_fix, P->nvox, "fixed-point accumulator"));
             RB_CHECK(P->alloc(&P->d_ht, P->nvox, "Ht"));
-            RB_CUDA(cudaMemset(P->d_fix, 0, P->nvox * sizeof(unsigned long long)));
             RB_CHECK(compat_alloc_volume(*P));
             RB_CHECK(build_compat_tables(*P, 0));
         }
@@ -677,7 +683,8 @@ recon_status_t recon_count_projector_pairs(recon_plan_t P, int projector, unsign
     if (projector != RECON_PROJECTOR_FORWARD && projector != RECON_PROJECTOR_BACK)
         return fail(RECON_ERR_INVALID_ARGUMENT, "projector must be RECON_PROJECTOR_FORWARD or RECON_PROJECTOR_BACK");
     RB_CHECK(use_device(*P));
-    if (projector == RECON_PROJECTOR_FORWARD && P->fp_column) return exact_fp_column_count(*P, count);
+    // (the ray design along detector columns walks as the column forward projector does)
+    if (P->fp_column && (projector == RECON_PROJECTOR_FORWARD || P->bp_columns)) return exact_fp_column_count(*P, count);
     if (projector == RECON_PROJECTOR_BACK && P->bp_gather) return exact_bp_gather_count(*P, count);
     return exact_count(*P, count);  // the ray walk, which these projectors run
 }

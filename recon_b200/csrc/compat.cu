@@ -496,25 +496,22 @@ __global__ void __launch_bounds__(kRayRows * kRayCols, 4) bp_scatter_kernel(
 }
 
 // Fixed point -> float (one rounding), then out = v (overwrite) or
-// out = out + v (siddon_add_bp into the running sum); the accumulator is
-// cleared for the next view.  The accumulator's z runs fastest, the image's x: 32 (x)
+// out = out + v (siddon_add_bp into the running sum).  The accumulator's z runs fastest, the image's x: 32 (x)
 // x 32 (z) tiles of one y through shared memory.
-__global__ void __launch_bounds__(256) bp_finish_kernel(unsigned long long* __restrict__ acc, int X, int Y, int Z,
+__global__ void __launch_bounds__(256) bp_finish_kernel(const unsigned long long* __restrict__ acc, int X, int Y, int Z,
                                                         const unsigned* __restrict__ maxabs, unsigned view, float chord,
                                                         int count_bits, float* __restrict__ out, int accumulate)
 {
     __shared__ float tile[32][33];
     const double scale = fix_scale(maxabs[view], chord, count_bits);
+    const double unscale = scale != 0.0 ? 1.0 / scale : 0.0;  // a power of two
     const int tx = (X + 31) / 32, x0 = (int)(blockIdx.x % tx) * 32, z0 = (int)(blockIdx.x / tx) * 32;
     for (int y = blockIdx.y; y < Y; y += gridDim.y) {
         for (int r = threadIdx.y; r < 32; r += 8) {
             const int x = x0 + r, z = z0 + threadIdx.x;
             float v = 0.0f;
-            if (scale != 0.0 && x < X && z < Z) {
-                unsigned long long* const a = acc + ((size_t)y * X + x) * Z + z;
-                v = (float)((double)(long long)*a / scale);
-                *a = 0ull;
-            }
+            if (scale != 0.0 && x < X && z < Z)
+                v = (float)((double)(long long)acc[((size_t)y * X + x) * Z + z] * unscale);
             tile[r][threadIdx.x] = v;
         }
         __syncthreads();
@@ -626,6 +623,7 @@ static recon_status_t launch_compat_bp(Plan& P, unsigned first, unsigned views, 
                                        unsigned slot, float chord, int cbits, float* out, bool accumulate,
                                        cudaStream_t s)
 {
+    RB_CUDA(cudaMemsetAsync(P.d_fix, 0, P.nvox * sizeof(unsigned long long), s));
     auto kernel = pow2_voxels(P) ? compat::bp_scatter_kernel<true> : compat::bp_scatter_kernel<false>;
     kernel<<<walk_grid(P, views), walk_block(), 0, s>>>(P.cg, P.d_angles, P.d_loopN, first, strides_z(P), img, img_stride,
                                                         P.d_maxabs, slot, chord, cbits, P.d_fix);

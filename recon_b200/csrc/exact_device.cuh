@@ -98,6 +98,30 @@ __device__ __forceinline__ float widen_hi(float2 x) { return x.y; }
 __device__ __forceinline__ float widen_lo(unsigned x) { return __uint_as_float(x << 16); }
 __device__ __forceinline__ float widen_hi(unsigned x) { return __uint_as_float(x & 0xffff0000u); }
 
+// A value as T stores it, in FP32.
+template <class T>
+__device__ __forceinline__ float as_stored(float v);
+template <>
+__device__ __forceinline__ float as_stored<float>(float v) { return v; }
+template <>
+__device__ __forceinline__ float as_stored<__nv_bfloat16>(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
+// *slot = max(*slot, the calling lanes' largest |value| as float bits): one atomic for the
+// active lanes of a warp, which nothing waits for.
+__device__ __forceinline__ void raise_max(unsigned* slot, float value)
+{
+    const unsigned active = __activemask();
+    const unsigned bits = __reduce_max_sync(active, __float_as_uint(fabsf(value)));
+    unsigned lane;
+    asm("mov.u32 %0, %%laneid;" : "=r"(lane));
+    if (bits && lane == (unsigned)__ffs(active) - 1u) atomicMax(slot, bits);
+}
+// The larger of two magnitudes as their float bits order them (NaN above infinity).
+__device__ __forceinline__ float max_bits(float a, float b)
+{
+    return __uint_as_float(max(__float_as_uint(fabsf(a)), __float_as_uint(fabsf(b))));
+}
+
 // ---- ray blocks ---------------------------------------------------------------------------
 
 // Rays are launched in blocks of 32 (u) x 4 (v).  A CTA's block comes from a
@@ -223,6 +247,24 @@ __device__ __forceinline__ int fix_exponent(unsigned maxabs_bits, float max_len,
     int e;
     frexp((double)m * (double)max_len, &e);
     return min(62 - count_bits - e, 120);
+}
+
+// The fixed-point scale of one call, worked out once for every thread that uses it:
+// 2^F (0 where nothing is to be summed), 2^-F, and whether a value was not finite.
+struct FixScale {
+    float scale;
+    int nonfinite;
+    double unscale;
+};
+
+__device__ __forceinline__ FixScale fix_scale_of(unsigned maxabs_bits, float max_len, int count_bits)
+{
+    const int F = fix_exponent(maxabs_bits, max_len, count_bits);
+    FixScale S;
+    S.scale = F == INT_MIN ? 0.0f : ldexpf(1.0f, F);
+    S.unscale = F == INT_MIN ? 0.0 : ldexp(1.0, -F);
+    S.nonfinite = !isfinite(__uint_as_float(maxabs_bits));
+    return S;
 }
 
 // One ray's contributions to the slab [k0, k1): cval = value * 2^F.  acc is

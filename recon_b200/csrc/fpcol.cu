@@ -141,6 +141,71 @@ __device__ __forceinline__ float walk_rows(const float* __restrict__ volz, const
     return acc + blk;
 }
 
+// Where a warp's rows start on the column path in spc (n pieces from t_in to t_out), for
+// detector row v of the calling lane: pieces jb..je (jb > je: no row of the warp crosses
+// the volume), and per lane as walk_rows takes it.  (column_row_sum has the same in
+// place: held at 32 registers, it spills through the struct.)  hit: the lane's row crosses the volume;
+// fast: no lane leaves it through the far face within the pieces.  Called by whole warps.
+struct RowWalk {
+    int jb, je, kaddr, dk, kexit;
+    float t_start, kf, tzn, S, O;
+    bool hit, fast;
+};
+
+__device__ __forceinline__ RowWalk row_walk(const ExactGeom& G, const ZParam* __restrict__ zp, const float2* spc, int n,
+                                            float t_in, float t_out, int v, bool valid)
+{
+    RowWalk W;
+    ZParam Z;
+    Z.S = 0.0f;
+    Z.O = 0.0f;
+    Z.inv_S = 0.0f;
+    Z.kc = 0;
+    if (valid) Z = zp[v];
+    W.S = Z.S;
+    W.O = Z.O;
+    // the volume's bottom and top planes along this row's ray
+    const float z0 = plane_t(0, Z.S, Z.O, Z.kc), zZ = plane_t(G.Z, Z.S, Z.O, Z.kc);
+    const float t_lo = fminf(z0, zZ), t_hi = fmaxf(z0, zZ);
+    const float ta = fmaxf(t_in, t_lo), tb = fminf(t_out, t_hi);
+    W.hit = valid && ta < tb;
+    W.jb = INT_MAX;
+    W.je = -1;
+    if (W.hit) {
+        W.jb = first_piece_ending<true>(spc, n, ta);
+        W.je = first_piece_ending<false>(spc, n, tb);
+    }
+    W.jb = __reduce_min_sync(0xffffffffu, W.jb);
+    W.je = __reduce_max_sync(0xffffffffu, W.je);
+    W.dk = Z.S > 0.0f ? 1 : -1;  // layer step along increasing t
+    W.kexit = W.dk > 0 ? G.Z + 1 : 0;
+    // rows that miss the volume read the zero layer below their column and never cross
+    W.kaddr = 0;
+    W.kf = 0.0f;
+    W.tzn = __int_as_float(0x7f800000);
+    W.t_start = 0.0f;
+    W.fast = true;
+    if (W.jb > W.je) return W;
+    W.t_start = (W.jb == 0) ? t_in : spc[W.jb - 1].x;
+    const float t_end = spc[W.je].x;
+    if (W.hit) {
+        int plane;  // the next z plane the row crosses
+        if (W.t_start < t_lo) {  // outside, the volume ahead: the first plane is the near face
+            W.kaddr = W.dk > 0 ? 0 : G.Z + 1;
+            plane = W.dk > 0 ? 0 : G.Z;
+        } else {  // inside (t_start <= ta < tb <= t_hi)
+            const int k = locate<true>(W.t_start, Z.S, Z.O, Z.kc, G.Z, 1.0 / (double)Z.S);
+            W.kaddr = k + 1;
+            plane = W.dk > 0 ? k + 1 : k;
+        }
+        W.kf = (float)(plane - Z.kc);
+        W.tzn = fmaf(W.kf, Z.S, Z.O);
+    }
+    const bool leaves = W.hit && W.t_start < t_hi && t_end > t_hi;  // crosses the far face within the pieces
+    W.fast = !__any_sync(0xffffffffu, leaves);
+    return W;
+}
+
 // Sum over the voxels that detector row v's ray crosses of (t_exit - t_entry) *
 // f[voxel] (the projection divided by w), for the column path in spc (n pieces
 // from t_in to t_out), or with COUNT the row's number of (ray, voxel) pairs.
@@ -299,99 +364,83 @@ __device__ __forceinline__ float2 walk_rows_mirror(const float* __restrict__ vol
     return make_float2(acc + blk, accm + blkm);
 }
 
-// column_row_sum for lower row v (v < Nv/2) and its mirror Nv-1-v.
-template <bool KAHAN, bool COUNT, bool PAIRED>
-__device__ __forceinline__ float2 column_row_sum_mirror(const ExactGeom& G, const ZParam* __restrict__ zp,
-                                                        const float* __restrict__ volz, const float2* spc, int n,
-                                                        float t_in, float t_out, int v, bool valid)
+// row_walk for lower row v (v < Nv/2), which descends along t (S < 0: its next plane is
+// the layer's own), and its mirror Nv-1-v.
+__device__ __forceinline__ RowWalk mirror_walk(const ExactGeom& G, const ZParam* __restrict__ zp, const float2* spc, int n,
+                                               float t_in, float t_out, int v, bool valid)
 {
+    RowWalk W;
     ZParam Z;
     Z.S = 0.0f;
     Z.O = 0.0f;
     Z.inv_S = 0.0f;
     Z.kc = 0;
     if (valid) Z = zp[v];
+    W.S = Z.S;
+    W.O = Z.O;
+    W.dk = -1;
+    W.kexit = 0;
     const float z0 = plane_t(0, Z.S, Z.O, Z.kc), zZ = plane_t(G.Z, Z.S, Z.O, Z.kc);
     const float t_lo = fminf(z0, zZ), t_hi = fmaxf(z0, zZ);  // the same for the mirror row
     const float ta = fmaxf(t_in, t_lo), tb = fminf(t_out, t_hi);
-    const bool hit = valid && ta < tb;
-    int jb = INT_MAX, je = -1;
-    if (hit) {
-        jb = first_piece_ending<true>(spc, n, ta);
-        je = first_piece_ending<false>(spc, n, tb);
+    W.hit = valid && ta < tb;
+    W.jb = INT_MAX;
+    W.je = -1;
+    if (W.hit) {
+        W.jb = first_piece_ending<true>(spc, n, ta);
+        W.je = first_piece_ending<false>(spc, n, tb);
     }
-    jb = __reduce_min_sync(0xffffffffu, jb);
-    je = __reduce_max_sync(0xffffffffu, je);
-    if (jb > je) return make_float2(0.0f, 0.0f);
-    const float t_start = (jb == 0) ? t_in : spc[jb - 1].x;
-    const float t_end = spc[je].x;
-    // lower rows descend along t (S < 0): their next plane is the layer's own
-    int kaddr = 0;
-    float kf = 0.0f, tzn = __int_as_float(0x7f800000);
-    if (hit) {
+    W.jb = __reduce_min_sync(0xffffffffu, W.jb);
+    W.je = __reduce_max_sync(0xffffffffu, W.je);
+    W.kaddr = 0;
+    W.kf = 0.0f;
+    W.tzn = __int_as_float(0x7f800000);
+    W.t_start = 0.0f;
+    W.fast = true;
+    if (W.jb > W.je) return W;
+    W.t_start = (W.jb == 0) ? t_in : spc[W.jb - 1].x;
+    const float t_end = spc[W.je].x;
+    if (W.hit) {
         int plane;
-        if (t_start < t_lo) {  // above the volume: the first plane is the top face
-            kaddr = G.Z + 1;
+        if (W.t_start < t_lo) {  // above the volume: the first plane is the top face
+            W.kaddr = G.Z + 1;
             plane = G.Z;
         } else {
-            const int k = locate<true>(t_start, Z.S, Z.O, Z.kc, G.Z, 1.0 / (double)Z.S);
-            kaddr = k + 1;
+            const int k = locate<true>(W.t_start, Z.S, Z.O, Z.kc, G.Z, 1.0 / (double)Z.S);
+            W.kaddr = k + 1;
             plane = k;
         }
-        kf = (float)(plane - Z.kc);
-        tzn = fmaf(kf, Z.S, Z.O);
+        W.kf = (float)(plane - Z.kc);
+        W.tzn = fmaf(W.kf, Z.S, Z.O);
     }
-    const bool leaves = hit && t_start < t_hi && t_end > t_hi;
-    if (!__any_sync(0xffffffffu, leaves))
-        return walk_rows_mirror<KAHAN, true, COUNT, PAIRED>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O,
-                                                            G.Z);
-    return walk_rows_mirror<KAHAN, false, COUNT, PAIRED>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, G.Z);
+    const bool leaves = W.hit && W.t_start < t_hi && t_end > t_hi;
+    W.fast = !__any_sync(0xffffffffu, leaves);
+    return W;
 }
 
-// MODE 0: out = projection (w * sum); MODE 1 (MLEM): out = w * g / Hf (0 where
-// Hf == 0), the Siddon back projector's input; MODE 2: out = g / Hf (the
-// voxel-driven back projector's); MODE 3: the (ray, voxel) pairs of positive
-// length are counted into out[0] (OT = unsigned long long); MODE 4: the sum is
-// added to out (float, detector-column layout), one xy block's share of it;
-// MODE 5: MODE 3 within one xy block.  MODES 4 and 5 take the column's stretch
-// inside the xy block blk = {x planes blk.x .. blk.y, y planes blk.z .. blk.w},
-// the others the whole volume's.
-// g is read [view][v][u]; out is written in LAYOUT: rows [view][v][u],
-// detector columns [view][u][v] (a warp's 32 rows store 128 contiguous bytes)
-// or, with MIRROR, mirrored row pairs (a lane stores its pair at once).  A CTA
-// takes detector column u of one view and rows vstart .. vstart + blockDim.x - 1:
-// from the tile list {view, u | vstart << 16} (blockIdx.x indexes it) or,
-// without one, u = blockIdx.x, vstart = blockIdx.y * blockDim.x, view = view0 +
-// blockIdx.z.
-// MIRROR: rows come in mirrored pairs (see walk_rows_mirror); the CTA's rows
-// are lower rows (below Nv/2) and each lane also produces its mirror row.
-template <bool KAHAN, int MODE, int LAYOUT, class GT, class OT, bool MIRROR = false>
-__device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out)
+// column_row_sum for lower row v (v < Nv/2) and its mirror Nv-1-v.
+template <bool KAHAN, bool COUNT, bool PAIRED>
+__device__ __forceinline__ float2 column_row_sum_mirror(const ExactGeom& G, const ZParam* __restrict__ zp,
+                                                        const float* __restrict__ volz, const float2* spc, int n,
+                                                        float t_in, float t_out, int v, bool valid)
 {
-    // piece j: {t where it ends, offset of its (x, y) voxel column in volz (int bits)}
-    extern __shared__ float2 spc[];
-    unsigned view;
-    int u, vstart;
-    if (tiles) {
-        const uint2 t = tiles[blockIdx.x];
-        view = t.x;
-        u = (int)(t.y & 0xffffu);
-        vstart = (int)(t.y >> 16);
-    } else {
-        view = view0 + blockIdx.z;
-        u = (int)blockIdx.x;
-        vstart = (int)(blockIdx.y * blockDim.x);
-    }
+    const RowWalk W = mirror_walk(G, zp, spc, n, t_in, t_out, v, valid);
+    if (W.jb > W.je) return make_float2(0.0f, 0.0f);
+    if (W.fast)
+        return walk_rows_mirror<KAHAN, true, COUNT, PAIRED>(volz, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S,
+                                                            W.O, G.Z);
+    return walk_rows_mirror<KAHAN, false, COUNT, PAIRED>(volz, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O,
+                                                         G.Z);
+}
+
+// The xy path of a detector column's rays from t_in to t_out inside the block b, by the
+// CTA's threads into spc (see the top of the file): its number of pieces, 0 when the rays
+// miss the block's footprint.  A barrier must follow.
+__device__ __forceinline__ int column_path(float2* spc, const ExactGeom& G, const float4 T, const int2 K, const int4 b,
+                                           float t_in, float t_out)
+{
     const int Zp = G.Z + 2;
-    const float4 T = __ldg(txy + (size_t)view * G.Nu + u);
-    const int2 K = __ldg(kxy + (size_t)view * G.Nu + u);
-    constexpr bool COUNTING = MODE == 3 || MODE == 5;
-    const int4 b = MODE >= 4 ? blk : make_int4(0, G.X, 0, G.Y);
-    const float x0 = plane_t(b.x, T.x, T.y, K.x), x1 = plane_t(b.y, T.x, T.y, K.x);
-    const float y0 = plane_t(b.z, T.z, T.w, K.y), y1 = plane_t(b.w, T.z, T.w, K.y);
-    const float t_in = fmaxf(fminf(x0, x1), fminf(y0, y1));
-    const float t_out = fminf(fmaxf(x0, x1), fmaxf(y0, y1));
-    int n = 0;  // pieces; 0 when the column's rays miss the block's xy footprint
+    int n = 0;
     if (t_in < t_out) {
         const double ivx = 1.0 / (double)T.x, ivy = 1.0 / (double)T.z;
         const int ix = locate_in<true>(t_in, T.x, T.y, K.x, b.x, b.y, ivx);
@@ -430,6 +479,53 @@ __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __
             spc[n - 1].x = fminf(fmaf((float)(qx + nx * dx), T.x, T.y), fmaf((float)(qy + ny * dy), T.z, T.w));
         }
     }
+    return n;
+}
+
+// MODE 0: out = projection (w * sum); MODE 1 (MLEM): out = w * g / Hf (0 where
+// Hf == 0), the Siddon back projector's input; MODE 2: out = g / Hf (the
+// voxel-driven back projector's); MODE 3: the (ray, voxel) pairs of positive
+// length are counted into out[0] (OT = unsigned long long); MODE 4: the sum is
+// added to out (float, detector-column layout), one xy block's share of it;
+// MODE 5: MODE 3 within one xy block.  MODES 4 and 5 take the column's stretch
+// inside the xy block blk = {x planes blk.x .. blk.y, y planes blk.z .. blk.w},
+// the others the whole volume's.
+// g is read [view][v][u]; out is written in LAYOUT: rows [view][v][u],
+// detector columns [view][u][v] (a warp's 32 rows store 128 contiguous bytes)
+// or, with MIRROR, mirrored row pairs (a lane stores its pair at once).  A CTA
+// takes detector column u of one view and rows vstart .. vstart + blockDim.x - 1:
+// from the tile list {view, u | vstart << 16} (blockIdx.x indexes it) or,
+// without one, u = blockIdx.x, vstart = blockIdx.y * blockDim.x, view = view0 +
+// blockIdx.z.
+// With vmax, MODE 1 raises vmax[view] to the largest |value| it writes (float bits).
+// MIRROR: rows come in mirrored pairs (see walk_rows_mirror); the CTA's rows
+// are lower rows (below Nv/2) and each lane also produces its mirror row.
+template <bool KAHAN, int MODE, int LAYOUT, class GT, class OT, bool MIRROR = false>
+__device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out, unsigned* __restrict__ vmax)
+{
+    // piece j: {t where it ends, offset of its (x, y) voxel column in volz (int bits)}
+    extern __shared__ float2 spc[];
+    unsigned view;
+    int u, vstart;
+    if (tiles) {
+        const uint2 t = tiles[blockIdx.x];
+        view = t.x;
+        u = (int)(t.y & 0xffffu);
+        vstart = (int)(t.y >> 16);
+    } else {
+        view = view0 + blockIdx.z;
+        u = (int)blockIdx.x;
+        vstart = (int)(blockIdx.y * blockDim.x);
+    }
+    const float4 T = __ldg(txy + (size_t)view * G.Nu + u);
+    const int2 K = __ldg(kxy + (size_t)view * G.Nu + u);
+    constexpr bool COUNTING = MODE == 3 || MODE == 5;
+    const int4 b = MODE >= 4 ? blk : make_int4(0, G.X, 0, G.Y);
+    const float x0 = plane_t(b.x, T.x, T.y, K.x), x1 = plane_t(b.y, T.x, T.y, K.x);
+    const float y0 = plane_t(b.z, T.z, T.w, K.y), y1 = plane_t(b.w, T.z, T.w, K.y);
+    const float t_in = fmaxf(fminf(x0, x1), fminf(y0, y1));
+    const float t_out = fminf(fmaxf(x0, x1), fmaxf(y0, y1));
+    const int n = column_path(spc, G, T, K, b, t_in, t_out);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int vend = MIRROR ? G.Nv / 2 : G.Nv;  // rows this kernel walks (mirrors come with them)
@@ -472,11 +568,14 @@ __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __
             OT* const o = out + ((size_t)(view - view0) * G.Nu + u) * Np * 2;
             const float a = value(v, sum.x), b = value(G.Nv - 1 - v, sum.y);
             store_pair<OT>(o + 2 * v, a, b);
+            if (MODE == 1 && vmax) raise_max(vmax + view, max_bits(as_stored<OT>(a), as_stored<OT>(b)));
             if (v == G.Nv / 2 - 1) store_pair<OT>(o + 2 * (v + 1), b, a);  // entry Nv/2: rows Nv/2, Nv/2 - 1
         } else {
             auto emit = [&](int row, float acc) {
-                const size_t pix = LAYOUT == kLayoutColumns ? (size_t)u * G.Nv + row : (size_t)row * G.Nu + u;
-                store_val<OT>(out + base + pix, value(row, acc));
+                const size_t pix = LAYOUT == kLayoutColumns ? base + (size_t)u * G.Nv + row : base + (size_t)row * G.Nu + u;
+                const float x = value(row, acc);
+                store_val<OT>(out + pix, x);
+                if (MODE == 1 && LAYOUT == kLayoutColumns && vmax) raise_max(vmax + view, as_stored<OT>(x));
             };
             emit(v, sum.x);
             if (MIRROR) emit(G.Nv - 1 - v, sum.y);
@@ -488,14 +587,14 @@ __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __
 // 2.98 against 3.07 ms at 256^3 / 360 / 512^2.  The xy-block walks (MODES 4, 5)
 // keep the compiler's own allocation, which measured faster for them.
 template <bool KAHAN, int MODE, int LAYOUT, class GT, class OT, bool MIRROR = false>
-__global__ void __launch_bounds__(kColRows, 16) fp_column_kernel(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out)
+__global__ void __launch_bounds__(kColRows, 16) fp_column_kernel(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out, unsigned* __restrict__ vmax)
 {
-    column_kernel_body<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>(G, txy, kxy, zp, wq, tiles, view0, blk, volz, g, out);
+    column_kernel_body<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>(G, txy, kxy, zp, wq, tiles, view0, blk, volz, g, out, vmax);
 }
 template <bool KAHAN, int MODE, int LAYOUT, class GT, class OT, bool MIRROR = false>
-__global__ void __launch_bounds__(kColRows) fp_column_block_kernel(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out)
+__global__ void __launch_bounds__(kColRows) fp_column_block_kernel(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out, unsigned* __restrict__ vmax)
 {
-    column_kernel_body<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>(G, txy, kxy, zp, wq, tiles, view0, blk, volz, g, out);
+    column_kernel_body<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>(G, txy, kxy, zp, wq, tiles, view0, blk, volz, g, out, vmax);
 }
 // the kernel of a MODE
 template <int MODE, bool KAHAN, int LAYOUT, class GT, class OT, bool MIRROR>
@@ -503,6 +602,180 @@ constexpr auto fp_column_kernel_of()
 {
     if constexpr (MODE >= 4) return fp_column_block_kernel<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>;
     else return fp_column_kernel<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>;
+}
+
+// ---- back projection along the same paths (the ray design's exact sums) ------------------
+//
+// A lane carries its row's value (times w and 2^F) along the path and adds every length
+// times it, rounded to an integer, to the 64-bit accumulator of the voxel it crosses (z
+// fastest, a layer of padding at each end that takes what lies outside): the products and
+// the sums of bp_ray_kernel (exact.cu) bit for bit, as integer sums do not depend on the
+// order.  The rows of a warp add to neighbouring addresses: about 10 sectors of L2 per warp
+// reduction against the slabs' 17, no slab walked twice, and the path found once for all
+// rows.  Bound by L2's atomics (61 % of its throughput at 200 x 200 x 120, 0.9e12 products
+// a second).  Per back projection, slabs to columns: 200 x 200 x 120 / 240 views in eight
+// subsets 2.83 -> 2.28 ms, 208^3 / 200 views 2.93 -> 1.64, 131 x 117 x 93 / 77 views 0.210 ->
+// 0.134.  (A gather of the same integers from values staged in shared memory won 1.3 to
+// 1.6 times where rows mirror and lie a voxel apart and lost elsewhere.)
+
+// One warp's rows over pieces jb..je; arguments as walk_rows.  With MIRROR the lane's lower
+// row and its mirror (value cvm, at offset Z + 1 - kaddr) share the lengths.
+template <bool FAST, int STEP, bool MIRROR>
+__device__ __forceinline__ void scatter_rows(unsigned long long* acc, const float2* spc, int jb, int je, float cur,
+                                             int kaddr, float kf, float tzn, float S, float O, int step, int kexit, int Z,
+                                             float cv, float cvm)
+{
+    const int st = STEP != 0 ? STEP : step;
+    const float fst = (float)st;
+    auto add = [](unsigned long long* p, float x) {
+        const long long q = __float2ll_rn(x);
+        if (q != 0) atomicAdd(p, (unsigned long long)q);
+    };
+#pragma unroll 4
+    for (int j = jb; j <= je; ++j) {
+        const float2 pc = spc[j];
+        const float B = pc.x;
+        unsigned long long* const col = acc + __float_as_int(pc.y);
+        const bool cross = tzn < B;
+        const float m = fminf(tzn, B), L0 = m - cur;
+        add(col + kaddr, L0 * cv);
+        if (MIRROR) add(col + (Z + 1 - kaddr), L0 * cvm);
+        if (cross) {
+            kaddr += st;
+            const float L1 = B - m;
+            add(col + kaddr, L1 * cv);
+            if (MIRROR) add(col + (Z + 1 - kaddr), L1 * cvm);
+            kf += fst;
+            tzn = fmaf(kf, S, O);
+            if (!FAST && kaddr == kexit) tzn = __int_as_float(0x7f800000);
+        }
+        cur = B;
+    }
+}
+
+// Detector columns as the forward kernel takes them (tiles, or the full grid from row v0).
+// vals: values times w in detector columns [view - view0][u][v], or with view_stride 0
+// one table for every view.
+template <bool MIRROR>
+__global__ void __launch_bounds__(kColRows) bp_column_kernel(ExactGeom G, const float4* __restrict__ txy,
+                                                             const int2* __restrict__ kxy, const ZParam* __restrict__ zp,
+                                                             const uint2* __restrict__ tiles, unsigned view0, int v0,
+                                                             const float* __restrict__ valsf,
+                                                             const __nv_bfloat16* __restrict__ valsb, size_t view_stride,
+                                                             const FixScale* __restrict__ fix,
+                                                             unsigned long long* __restrict__ acc)
+{
+    extern __shared__ float2 spc[];
+    unsigned view;
+    int u, vstart;
+    if (tiles) {
+        const uint2 t = tiles[blockIdx.x];
+        view = t.x;
+        u = (int)(t.y & 0xffffu);
+        vstart = (int)(t.y >> 16);
+    } else {
+        view = view0 + blockIdx.z;
+        u = (int)blockIdx.x;
+        vstart = v0 + (int)(blockIdx.y * blockDim.x);
+    }
+    const int vend = MIRROR ? G.Nv / 2 : G.Nv;
+    const int v = vstart + (int)threadIdx.x;
+    const bool valid = v < vend;
+    // the value(s) of the lane's row(s): every load before any is used
+    const size_t pc = (size_t)(view - view0) * view_stride + (size_t)u * G.Nv;
+    float x = 0.0f, xm = 0.0f;
+    if (valid) {
+        x = valsf ? __ldg(valsf + pc + v) : load_val<__nv_bfloat16>(valsb + pc + v);
+        if (MIRROR) xm = valsf ? __ldg(valsf + pc + (G.Nv - 1 - v)) : load_val<__nv_bfloat16>(valsb + pc + (G.Nv - 1 - v));
+    }
+    const float scale = __ldg(&fix->scale);
+    if (scale == 0.0f) return;  // the whole block: all zero or not finite
+    const float4 T = __ldg(txy + (size_t)view * G.Nu + u);
+    const int2 K = __ldg(kxy + (size_t)view * G.Nu + u);
+    const int4 b = make_int4(0, G.X, 0, G.Y);
+    const float x0 = plane_t(b.x, T.x, T.y, K.x), x1 = plane_t(b.y, T.x, T.y, K.x);
+    const float y0 = plane_t(b.z, T.z, T.w, K.y), y1 = plane_t(b.w, T.z, T.w, K.y);
+    const float t_in = fmaxf(fminf(x0, x1), fminf(y0, y1));
+    const float t_out = fminf(fmaxf(x0, x1), fmaxf(y0, y1));
+    const int n = column_path(spc, G, T, K, b, t_in, t_out);
+    __syncthreads();
+    if (n == 0 || v - (int)(threadIdx.x & 31u) >= vend) return;  // whole warps
+    const float cv = x * scale, cvm = xm * scale;
+    const RowWalk W = MIRROR ? mirror_walk(G, zp, spc, n, t_in, t_out, v, valid && (cv != 0.0f || cvm != 0.0f))
+                             : row_walk(G, zp, spc, n, t_in, t_out, v, valid && cv != 0.0f);
+    if (W.jb > W.je) return;  // no row of the warp crosses the volume with a value
+    const float a = W.hit ? cv : 0.0f, am = W.hit ? cvm : 0.0f;
+    if (MIRROR) {
+        if (W.fast) scatter_rows<true, -1, true>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, -1, 0, G.Z, a, am);
+        else scatter_rows<false, -1, true>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, -1, 0, G.Z, a, am);
+    } else if (W.fast) {
+        scatter_rows<true, 0, false>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, W.dk, W.kexit, G.Z, a, am);
+    } else {
+        scatter_rows<false, 0, false>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, W.dk, W.kexit, G.Z, a, am);
+    }
+}
+
+// The result from the accumulator (z fastest, padded): 32 (x) x 32 (z) tiles of one y
+// through shared memory.  (Clearing it here, behind the loads, took 264 us at 256^3
+// against 41 us without and 28 us for a memset before the next sums.)  MODE 0: vol = Ht; MODE 2: the MLEM update, as
+// bp_finish_kernel (exact.cu).
+template <int MODE>
+__global__ void __launch_bounds__(256) bp_column_finish_kernel(ExactGeom G, const FixScale* __restrict__ fix,
+                                                               const unsigned long long* __restrict__ acc,
+                                                               float* __restrict__ vol, const float* __restrict__ sens)
+{
+    __shared__ float tile[32][33];
+    const bool nonfinite = __ldg(&fix->nonfinite);  // a non-finite input value makes every voxel NaN
+    const double unscale = __ldg(&fix->unscale);
+    const int tx = (G.X + 31) / 32, x0 = (int)(blockIdx.x % tx) * 32, z0 = (int)(blockIdx.x / tx) * 32;
+    for (int y = blockIdx.y; y < G.Y; y += gridDim.y) {
+        unsigned long long q[4];
+        float f[4], sv[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int x = x0 + threadIdx.y + 8 * r, z = z0 + threadIdx.x;
+            q[r] = (x < G.X && z < G.Z) ? acc[((size_t)y * G.X + x) * (G.Z + 2) + z + 1] : 0ull;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int x = x0 + threadIdx.x, z = z0 + threadIdx.y + 8 * r;
+            const bool in = MODE == 2 && x < G.X && z < G.Z;
+            const size_t v = ((size_t)z * G.Y + y) * G.X + x;
+            f[r] = in ? vol[v] : 0.0f;
+            sv[r] = in ? sens[v] : 0.0f;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int x = x0 + threadIdx.y + 8 * r, z = z0 + threadIdx.x;
+            tile[threadIdx.y + 8 * r][threadIdx.x] =
+                nonfinite ? __int_as_float(0x7fffffff) : (float)((double)(long long)q[r] * unscale);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int x = x0 + threadIdx.x, z = z0 + threadIdx.y + 8 * r;
+            if (x >= G.X || z >= G.Z) continue;
+            const float ht = tile[threadIdx.x][threadIdx.y + 8 * r];
+            const size_t v = ((size_t)z * G.Y + y) * G.X + x;
+            vol[v] = MODE == 2 ? ((sv[r] != 0.0f) ? __fdiv_rn(__fmul_rn(f[r], ht), sv[r]) : 0.0f) : ht;
+        }
+        __syncthreads();
+    }
+}
+
+// The call's scale from its views' maxima m[0 .. n).
+__global__ void fix_scale_kernel(const unsigned* __restrict__ m, unsigned n, float max_len, int count_bits,
+                                 FixScale* __restrict__ out)
+{
+    __shared__ unsigned top;
+    if (threadIdx.x == 0) top = 0u;
+    __syncthreads();
+    unsigned v = 0u;
+    for (unsigned q = threadIdx.x; q < n; q += blockDim.x) v = max(v, m[q]);
+    v = __reduce_max_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31u) == 0u) atomicMax(&top, v);
+    __syncthreads();
+    if (threadIdx.x == 0) *out = fix_scale_of(top, max_len, count_bits);
 }
 
 // f[z][y][x] -> volz[(y*X + x)*(Z + 2) + z + 1], 32 (x) x 32 (z) tiles of one y
@@ -558,7 +831,8 @@ __global__ void __launch_bounds__(128) column_block_mask_kernel(ExactGeom G, con
 template <int MODE, int LAYOUT, class GT, class OT>
 __global__ void __launch_bounds__(256) column_finish_kernel(ExactGeom G, const float* acc,
                                                             const float* __restrict__ wq,
-                                                            const GT* __restrict__ g, OT* out)
+                                                            const GT* __restrict__ g, OT* out,
+                                                            unsigned* __restrict__ vmax)
 {
     __shared__ float tile[32][33];
     const int u0 = blockIdx.x * 32, v0 = blockIdx.y * 32;
@@ -585,7 +859,10 @@ __global__ void __launch_bounds__(256) column_finish_kernel(ExactGeom G, const f
                 const float ratio = (hf != 0.0f) ? __fdiv_rn(tile[threadIdx.x][threadIdx.y + 8 * q], hf) : 0.0f;
                 val[q] = MODE == 1 ? ratio * w : ratio;
             }
-            if (LAYOUT == kLayoutColumns) store_val<OT>(out + base + pc, val[q]);
+            if (LAYOUT == kLayoutColumns) {
+                store_val<OT>(out + base + pc, val[q]);
+                if (MODE == 1 && vmax) raise_max(vmax + blockIdx.z, as_stored<OT>(val[q]));
+            }
         }
     }
     if (LAYOUT == kLayoutRows) {
@@ -607,7 +884,8 @@ __global__ void __launch_bounds__(256) column_finish_kernel(ExactGeom G, const f
 template <int MODE, class GT, class OT>
 __global__ void __launch_bounds__(256) column_finish_pairs_kernel(ExactGeom G, const float* __restrict__ acc,
                                                                   const float* __restrict__ wq,
-                                                                  const GT* __restrict__ g, OT* __restrict__ out)
+                                                                  const GT* __restrict__ g, OT* __restrict__ out,
+                                                                  unsigned* __restrict__ vmax)
 {
     __shared__ float lo[32][33], hi[32][33];
     const int Np = G.Nv / 2 + 1;  // pairs; a column holds pair_entries(Nv) entries
@@ -638,6 +916,7 @@ __global__ void __launch_bounds__(256) column_finish_pairs_kernel(ExactGeom G, c
         const float a = value(p, MODE ? lo[threadIdx.x][threadIdx.y + 8 * q] : 0.0f);
         const float b = value(G.Nv - 1 - p, MODE ? hi[threadIdx.x][threadIdx.y + 8 * q] : 0.0f);
         store_pair<OT>(out + (((size_t)blockIdx.z * G.Nu + u) * pair_entries(G.Nv) + p) * 2, a, b);
+        if (MODE == 1 && vmax) raise_max(vmax + blockIdx.z, max_bits(as_stored<OT>(a), as_stored<OT>(b)));
     }
 }
 
@@ -824,6 +1103,13 @@ static auto column_kernel(const Plan& P)
     }
 }
 
+// Where the ray design finds the ratio's largest |value| of views first, ...
+template <int MODE>
+static unsigned* ratio_max(const Plan& P, unsigned first)
+{
+    return (MODE == 1 && P.bp_columns) ? P.d_vmax + first : nullptr;
+}
+
 // Views [first, first + count) of plan views over the xy blocks: each block's
 // tiles add their stretch of the ray sums into acc (in launch order, so the sums
 // are deterministic), then column_finish_kernel forms the output; MODE 3 adds
@@ -862,17 +1148,19 @@ static recon_status_t launch_column_blocks(Plan& P, const float* vol, unsigned f
             if (nt == 0) continue;
             const int4 blk = make_int4(bx * side, std::min((bx + 1) * side, E.X), by * side,
                                        std::min((by + 1) * side, E.Y));
-            kernel<<<nt, P.col_rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, P.d_wq, T.d + t0, first, blk,
-                                                     P.d_vol_z, nullptr, bout);
+            kernel<<<nt, P.col_rows, smem, s>>>(P.eg, P.d_txy, P.d_kxy, P.d_zp, P.d_wq, T.d + t0, first, blk,
+                                                     P.d_vol_z, nullptr, bout, nullptr);
             RB_CUDA(cudaGetLastError());
         }
     if constexpr (MODE != 3 && LAYOUT == kLayoutPairs) {
         const dim3 grid((E.Nu + 31) / 32, (E.Nv / 2 + 1 + 31) / 32, count);
-        exact::column_finish_pairs_kernel<MODE, GT, OT><<<grid, dim3(32, 8), 0, s>>>(E, acc, P.d_wq, g, out);
+        exact::column_finish_pairs_kernel<MODE, GT, OT><<<grid, dim3(32, 8), 0, s>>>(E, acc, P.d_wq, g, out,
+                                                                                    ratio_max<MODE>(P, first));
         RB_CUDA(cudaGetLastError());
     } else if constexpr (MODE != 3) {
         const dim3 grid((E.Nu + 31) / 32, (E.Nv + 31) / 32, count);
-        exact::column_finish_kernel<MODE, LAYOUT, GT, OT><<<grid, dim3(32, 8), 0, s>>>(E, acc, P.d_wq, g, out);
+        exact::column_finish_kernel<MODE, LAYOUT, GT, OT><<<grid, dim3(32, 8), 0, s>>>(E, acc, P.d_wq, g, out,
+                                                                                      ratio_max<MODE>(P, first));
         RB_CUDA(cudaGetLastError());
     }
     return RECON_OK;
@@ -890,6 +1178,7 @@ static recon_status_t launch_column(Plan& P, const float* vol, unsigned first, u
     if (count == 0) return RECON_OK;
     const ExactGeom& E = P.eg;
     const bool plan_views = first + count <= P.nviews;
+    if (unsigned* m = ratio_max<MODE>(P, first)) RB_CUDA(cudaMemsetAsync(m, 0, count * sizeof(unsigned), s));
     if (plan_views && P.col_block > 0 && P.col_btiles.size() == (size_t)P.col_nbx * P.col_nby)
         return launch_column_blocks<MODE, LAYOUT, GT, OT>(P, vol, first, count, g, out, s);
     dim3 grid;
@@ -909,10 +1198,60 @@ static recon_status_t launch_column(Plan& P, const float* vol, unsigned first, u
     auto kernel = column_kernel<MODE, LAYOUT, GT, OT>(P);
     if (smem > 48 * 1024) RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<grid, P.col_rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, P.d_wq, tiles, first,
-                                               make_int4(0, E.X, 0, E.Y), P.d_vol_z, g, out);
+                                               make_int4(0, E.X, 0, E.Y), P.d_vol_z, g, out, ratio_max<MODE>(P, 0));
     RB_CUDA(cudaGetLastError());
     return RECON_OK;
 }
+
+// The ray design's back projection along detector columns: views [first, first + count) of
+// table slots, vals their values times w in detector columns (view_stride 0: one table for
+// every view), vmax[0 .. nmax) the views' largest magnitudes; vol = Ht, or with sens the
+// MLEM update of vol.
+template <class ST>
+recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, unsigned first, unsigned count,
+                          const unsigned* vmax, unsigned nmax, float* vol, const float* sens, cudaStream_t s)
+{
+    const ExactGeom& E = P.eg;
+    RB_CUDA(cudaMemsetAsync(P.d_bpacc, 0, bp_acc_words(P) * sizeof(unsigned long long), s));
+    exact::FixScale* const fix = reinterpret_cast<exact::FixScale*>(P.d_bpmax);
+    exact::fix_scale_kernel<<<1, 256, 0, s>>>(vmax, nmax, bp_max_len(P), bp_count_bits(P, count), fix);
+    RB_CUDA(cudaGetLastError());
+    const size_t smem = (size_t)(E.X + E.Y + 2) * sizeof(float2);
+    auto kernel = P.z_mirror ? exact::bp_column_kernel<true> : exact::bp_column_kernel<false>;
+    if (smem > 48 * 1024) RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const float* vf = nullptr;
+    const __nv_bfloat16* vb = nullptr;
+    if constexpr (std::is_same<ST, float>::value) vf = vals;
+    else vb = vals;
+    auto launch = [&](dim3 grid, int rows, const uint2* tiles, int v0) -> recon_status_t {
+        kernel<<<grid, rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, tiles, first, v0, vf, vb, view_stride, fix, P.d_bpacc);
+        RB_CUDA(cudaGetLastError());
+        return RECON_OK;
+    };
+    const int rows = P.z_mirror ? E.Nv / 2 : E.Nv;
+    if (count > 24 && bp_acc_words(P) * sizeof(unsigned long long) > (size_t(115) << 20)) {
+        // an accumulator that the 126 MB L2 does not hold: 32 rows of every view at a time,
+        // whose rays meet a slab of it (256^3, 120 views: 3.45 against 5.4 ms by views; at
+        // 240^3, 113 MB, by views 2.8 against 2.95 ms; ten views are faster by views)
+        for (int v0 = 0; v0 < rows; v0 += 32) RB_CHECK(launch(dim3(E.Nu, 1, count), 32, nullptr, v0));
+    } else if (first + count <= P.nviews && P.col_tiles.prefix.size() == P.nviews + 1) {
+        const unsigned t0 = P.col_tiles.prefix[first], nt = P.col_tiles.prefix[first + count] - t0;
+        if (nt) RB_CHECK(launch(dim3(nt, 1, 1), P.col_rows, P.col_tiles.d + t0, 0));
+    } else {
+        RB_CHECK(launch(dim3(E.Nu, (rows + P.col_rows - 1) / P.col_rows, count), P.col_rows, nullptr, 0));
+    }
+    const dim3 fgrid((unsigned)((E.X + 31) / 32) * (unsigned)((E.Z + 31) / 32), std::min(E.Y, 65535));
+    if (sens)
+        exact::bp_column_finish_kernel<2><<<fgrid, dim3(32, 8), 0, s>>>(E, fix, P.d_bpacc, vol, sens);
+    else
+        exact::bp_column_finish_kernel<0><<<fgrid, dim3(32, 8), 0, s>>>(E, fix, P.d_bpacc, vol, sens);
+    RB_CUDA(cudaGetLastError());
+    return RECON_OK;
+}
+template recon_status_t bp_columns<float>(Plan&, const float*, size_t, unsigned, unsigned, const unsigned*, unsigned,
+                                          float*, const float*, cudaStream_t);
+template recon_status_t bp_columns<__nv_bfloat16>(Plan&, const __nv_bfloat16*, size_t, unsigned, unsigned, const unsigned*,
+                                                  unsigned, float*, const float*, cudaStream_t);
 
 // (ray, voxel) pairs of positive length over all plan views, as the column
 // kernel assigns them (synchronous; no volume is read).

@@ -96,5 +96,4 @@ template <int EPI, class ST>
 recon_status_t staged_quarter_gather(Plan& P, const ST* vals, size_t view_stride, float* vol, const float* sens,
                                      cudaStream_t s, unsigned long long* npairs, bool set, unsigned m0, unsigned mc,
                                      bool* served);
-
 }  // namespace rb

@@ -18,11 +18,7 @@
 // limit), TMA boxes 2.10, two or four views to a stage instead of one 1.75, packed
 // multiply-adds without a predicate 1.56.  Reading the zero entry of a region in place
 // of the predicate cost bank conflicts (2.05).
-#include "exact_device.cuh"
-#include "gather_device.cuh"
-#include "internal.h"
-
-#include <cudaTypedefs.h>
+#include "gather_staged.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -31,80 +27,6 @@
 namespace rb {
 namespace exact {
 
-// What a stage holds and how columns meet the detector, from the host (staged_shape).
-struct StagedShape {
-    int rows;     // staged entries per detector column (multiple of 4): the box's width
-    int cols;     // staged detector columns per view: the box's height
-    int stages;   // stages in flight
-    int wide;     // most detector columns one voxel column meets in a view: 1, 2, 4 or 8
-};
-
-// One detector column of one view as a voxel column sees it: the piece [A, B] of
-// its rays, row coefficients ca = ez / (A + Rf), cb = ez / (B + Rf), their steps
-// per slot (32 voxels) pa, pb, and the detector column u; one = no voxel of the
-// column has a second candidate row there.
-struct StagedItem {
-    float A, B, pa, pb, ca, cb;
-    int u, one;
-};
-
-// ---- bulk copies and their barriers --------------------------------------------------------
-
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned bar)
-{
-    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes)
-{
-    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(bar),
-                 "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity)
-{
-    unsigned done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity), "r"(1000000u)  // the warp may sleep up to 1 ms (ns) in one try
-        : "memory");
-    return done != 0u;
-}
-// Waits until the barrier's phase of this parity is complete; gives up after about
-// two seconds (false), which no run that works comes near.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity)
-{
-    if (mbar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try(bar, parity))
-        if (clock64() - t0 > 4000000000ll) return false;
-    return true;
-}
-// The box at entry x (a multiple of four) of table row y into dst (128-byte aligned).
-__device__ __forceinline__ void tile_load(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            dst),
-        "l"(map), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-
-// a += L * x in both halves: one packed instruction, each half rounded as fmaf.
-__device__ __forceinline__ void fma_pair(float2& a, float L, float2 x)
-{
-    unsigned long long acc = *reinterpret_cast<unsigned long long*>(&a);
-    const unsigned long long v = *reinterpret_cast<const unsigned long long*>(&x);
-    asm("{\n\t.reg .b64 l;\n\tmov.b64 l, {%1, %1};\n\tfma.rn.f32x2 %0, l, %2, %0;\n\t}" : "+l"(acc) : "f"(L), "l"(v));
-    a = *reinterpret_cast<float2*>(&acc);
-}
-
 // ---- the quarter-turn gather ----------------------------------------------------------------
 
 // bp_gather_quarter_kernel's sums (see there: one warp per base column of the
@@ -112,96 +34,7 @@ __device__ __forceinline__ void fma_pair(float2& a, float L, float2 x)
 // four columns of its orbit at views m + rQ), in the same order, so the same bits.
 // A CTA owns TX x TY base columns (kWarps warps) and a loading warp; a stage holds
 // the four views' values of one base view, [r][detector column][row pair].
-constexpr int kStagedTX = 4, kStagedTY = 4;
-constexpr int kStagedWarps = kStagedTX * kStagedTY;
-constexpr int kStagedThreads = (kStagedWarps + 1) * 32;
 constexpr int kStageBytes = 98304;  // a stage: two or four base views of four regions of 12 or 6 KiB
-
-// Reads of shared memory at 32-bit addresses: a pair as stored (widen_lo / widen_hi
-// give its values), a row's z planes.
-__device__ __forceinline__ float2 lds_pair(unsigned a, float)
-{
-    float2 p;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(p.x), "=f"(p.y) : "r"(a));
-    return p;
-}
-__device__ __forceinline__ unsigned lds_pair(unsigned a, __nv_bfloat16)
-{
-    unsigned p;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(p) : "r"(a));
-    return p;
-}
-__device__ __forceinline__ float4 lds_planes(unsigned a)
-{
-    float4 p;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(a));
-    return p;
-}
-
-// Sum of |a| d / ... : the rows (relative to row 0) that heights [zb, zt] can be
-// seen at from depths [dmin, dmax], widened by one row.
-__device__ __forceinline__ void staged_rows(const GatherConst& C, float zb, float zt, float dmin, float dmax,
-                                            float& lo, float& hi)
-{
-    const float b0 = zb / dmin * C.ez, b1 = zb / dmax * C.ez, t0 = zt / dmin * C.ez, t1 = zt / dmax * C.ez;
-    lo = fminf(b0, b1) + C.oz - 1.0f;
-    hi = fmaxf(t0, t1) + C.oz + 1.0f;
-}
-
-// The first detector column that the rectangle [Xa, Xb] x [Ya, Yb] shadows at a view;
-// the columns that staged_item gives a voxel column inside it start there or later.
-__device__ __forceinline__ int staged_first_column(const ExactGeom& G, const GatherConst& C, const float2 CS, float Xa,
-                                                   float Xb, float Ya, float Yb)
-{
-    float umin = 3.0e38f;
-#pragma unroll
-    for (int c4 = 0; c4 < 4; ++c4) {
-        const float X = (c4 & 1) ? Xb : Xa, Y = (c4 & 2) ? Yb : Ya;
-        const float a = X * CS.x - Y * CS.y, b = X * CS.y + Y * CS.x;
-        umin = fminf(umin, __fdividef(a, b + G.Rf) * C.eu + C.ou);
-    }
-    return min(max(0, __float2int_ru(umin - 0.02f)), G.Nu - 1);
-}
-
-// Voxel column (i, j)'s item for detector column number sl of its range at a view;
-// valid when it returns true.
-__device__ __forceinline__ bool staged_item(const ExactGeom& G, const GatherConst& C, const float4* __restrict__ txy,
-                                            const int2* __restrict__ kxy, const float2 CS, unsigned view, int sl, int i,
-                                            int j, float Xa, float Xb, float Ya, float Yb, float margin, float dz32,
-                                            StagedItem& it)
-{
-    float umin = 3.0e38f, umax = -3.0e38f;
-#pragma unroll
-    for (int c4 = 0; c4 < 4; ++c4) {
-        const float X = (c4 & 1) ? Xb : Xa, Y = (c4 & 2) ? Yb : Ya;
-        const float a = X * CS.x - Y * CS.y, b = X * CS.y + Y * CS.x;
-        const float uf = __fdividef(a, b + G.Rf) * C.eu + C.ou;
-        umin = fminf(umin, uf);
-        umax = fmaxf(umax, uf);
-    }
-    const int u_lo = min(max(0, __float2int_ru(umin - 0.01f)), G.Nu);
-    const int u_hi = min(G.Nu - 1, __float2int_rd(umax + 0.01f));
-    it.u = u_lo + sl;
-    if (it.u > u_hi) return false;
-    const float4 T = __ldg(txy + (size_t)view * G.Nu + it.u);
-    const int2 K = __ldg(kxy + (size_t)view * G.Nu + it.u);
-    const float xa = plane_t(i, T.x, T.y, K.x), xb = plane_t(i + 1, T.x, T.y, K.x);
-    const float ya = plane_t(j, T.z, T.w, K.y), yb = plane_t(j + 1, T.z, T.w, K.y);
-    it.A = fmaxf(fminf(xa, xb), fminf(ya, yb));
-    it.B = fminf(fmaxf(xa, xb), fmaxf(ya, yb));
-    if (!(it.A < it.B)) return false;
-    it.ca = __fdividef(C.ez, it.A + G.Rf);
-    it.cb = __fdividef(C.ez, it.B + G.Rf);
-    it.pa = dz32 * it.ca;
-    it.pb = dz32 * it.cb;
-    // a voxel's candidate interval has a length convex in its height, largest at
-    // the column's bottom or top voxel
-    const float zb = G.P0[2], zt = G.P0[2] + (float)G.Z * G.vox[2];
-    const float len_b = fmaxf((zb + G.vox[2]) * it.ca, (zb + G.vox[2]) * it.cb) - fminf(zb * it.ca, zb * it.cb);
-    const float len_t = fmaxf(zt * it.ca, zt * it.cb) - fminf((zt - G.vox[2]) * it.ca, (zt - G.vox[2]) * it.cb);
-    it.one = (fmaxf(len_b, len_t) + margin < 0.99f) ? 1 : 0;
-    return true;
-}
 
 template <int EPI, class ST, int PS, int RB, bool SET>
 __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
@@ -492,14 +325,12 @@ static int staged_span(const Plan& P, double d, double rad)
     return (int)std::floor(d / dmin * std::sqrt(1.0 + tan * tan) * std::fabs((double)E.Ry / E.du) + 0.05) + 1;
 }
 
-// The stage layout for chunks of 32 * slots slices of the lower half, or false where the
-// staged gather does not serve and bp_gather_quarter_kernel does: a volume that comes
-// near the source (a piece could then lie behind it), a voxel column that meets more than
-// eight detector columns, a box of more than 256 a side or 12 KiB (a detector several
-// times finer than the voxels: its rows and columns then outgrow the two stages that a
-// block's shared memory holds).
-static bool staged_shape(const Plan& P, int slots, size_t value_bytes, exact::StagedShape* out, int* region,
-                         size_t* smem)
+// The boxes that tiles read in chunks of 32 * slots of Zs slices, of a detector whose
+// columns have entries 0 .. top (in multiples of `align` entries): S->wide, cols and rows.
+// False where no staged gather serves: a volume that comes near the source (a piece could
+// then lie behind it), a voxel column that meets more than eight detector columns, or a
+// box of more than 256 a side.
+bool staged_boxes(const Plan& P, int slots, int Zs, int top, int align, exact::StagedShape* S)
 {
     const ExactGeom& E = P.eg;
     const double vx = E.vox[0], vy = E.vox[1], vz = E.vox[2];
@@ -507,36 +338,44 @@ static bool staged_shape(const Plan& P, int slots, size_t value_bytes, exact::St
     const double rad = std::hypot(0.5 * E.X * vx + tx, 0.5 * E.Y * vy + ty) * 1.001;
     if (!(rad < 0.9 * (double)E.Rf)) return false;
     const double ez = (double)E.Ry / E.dv, oz = -((double)E.Dz + E.vd0) / E.dv;
-    exact::StagedShape S;
     const int wide = staged_span(P, std::hypot(vx, vy), rad);
     if (wide > 8) return false;
-    S.wide = wide <= 1 ? 1 : wide <= 2 ? 2 : wide <= 4 ? 4 : 8;
-    S.cols = staged_span(P, std::hypot(tx, ty), rad);
-    const int Zh = E.Z / 2, Nh = E.Nv / 2;
-    int rows = 0;
-    for (int k0 = 0; k0 < Zh; k0 += 32 * slots) {
-        const double zb = E.P0[2] + k0 * vz, zt = E.P0[2] + std::min(k0 + 32 * slots, Zh) * vz;
+    S->wide = wide <= 1 ? 1 : wide <= 2 ? 2 : wide <= 4 ? 4 : 8;
+    S->cols = staged_span(P, std::hypot(tx, ty), rad);
+    int rows = align;
+    for (int k0 = 0; k0 < Zs; k0 += 32 * slots) {
+        const double zb = E.P0[2] + k0 * vz, zt = E.P0[2] + std::min(k0 + 32 * slots, Zs) * vz;
         const double dn = E.Rf - rad, df = E.Rf + rad;
         const double lo = std::min(zb / dn * ez, zb / df * ez) + oz - 2.0;
         const double hi = std::max(zt / dn * ez, zt / df * ez) + oz + 2.0;
-        const int a = std::max(0, (int)std::floor(lo)) & ~3, b = std::min(Nh, (int)std::ceil(hi));
-        rows = std::max(rows, ((b - a + 1) + 3) / 4 * 4);
+        if (!(lo > -1e8 && hi < 1e8)) return false;
+        const int a = std::min(std::max(0, (int)std::floor(lo)), top) / align * align;
+        const int b = std::max(a, std::min(top, (int)std::ceil(hi)));
+        rows = std::max(rows, (b - a + align) / align * align);
     }
-    S.rows = std::max(rows, 4);
-    if (S.rows > 256 || S.cols > 256) return false;  // a box's sides
-    const size_t pair = 2 * value_bytes;
-    const size_t used = (size_t)S.cols * S.rows * pair;
+    S->rows = rows;
+    return S->rows <= 256 && S->cols <= 256;
+}
+
+// The quarter-turn kernel's stages for chunks of 32 * slots slices of the lower half, or
+// false where bp_gather_quarter_kernel is the quarter-turn gather instead: no boxes, or
+// boxes of more than 12 KiB (a detector several times finer than the voxels: its rows and
+// columns then outgrow the two stages that a block's shared memory holds).
+static bool staged_shape(const Plan& P, int slots, size_t value_bytes, exact::StagedShape* out, int* region,
+                         size_t* smem)
+{
+    exact::StagedShape S{};
+    if (!staged_boxes(P, slots, P.eg.Z / 2, P.eg.Nv / 2, 4, &S)) return false;
+    const size_t used = (size_t)S.cols * S.rows * 2 * value_bytes;
     if (used > 12288) return false;
     *region = used <= 6144 ? 6144 : 12288;
     const size_t planes = ((size_t)S.rows * sizeof(float4) + 127) / 128 * 128;
-    const size_t stage = exact::kStageBytes;
     const size_t epilogue = sizeof(float) * exact::kStagedWarps * 8 * slots * 32;
-    const size_t fixed = sizeof(exact::StagedItem) * 32 * exact::kStagedWarps + 1024;  // static shared memory
-    const size_t room = 227 * 1024 - fixed - planes;
-    if (planes + fixed > 100 * 1024 || 2 * stage > room || epilogue > room) return false;
-    S.stages = (int)std::min<size_t>(4, room / stage);
+    const size_t room = kStagedSmem - planes;
+    if (2 * (size_t)exact::kStageBytes > room || epilogue > room) return false;
+    S.stages = (int)std::min<size_t>(4, room / exact::kStageBytes);
     *out = S;
-    *smem = 128 + planes + std::max((size_t)S.stages * stage, epilogue);  // 128: the base's alignment
+    *smem = 128 + planes + std::max((size_t)S.stages * exact::kStageBytes, epilogue);  // 128: the base's alignment
     return true;
 }
 
@@ -554,19 +393,23 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     return fn;
 }
 
-// Mirrored row pairs as a table of `table_rows` detector columns of pair_entries(Nv)
-// entries (an entry is moved as one 8- or 4-byte element), read in boxes of S.rows
-// entries x S.cols detector columns.
-static bool pair_map(const Plan& P, const exact::StagedShape& S, const void* vals, size_t pair_bytes, size_t table_rows,
-                     CUtensorMap* map)
+bool staged_maps_available() { return tensor_map_encoder() != nullptr; }
+
+// A table of `table_rows` detector columns of `pitch` entries (a row pair, or a value; an
+// entry is moved as one element of `entry` bytes), read in boxes of S.rows entries x S.cols
+// detector columns.
+bool column_map(const exact::StagedShape& S, const void* vals, size_t pitch, size_t entry, size_t table_rows,
+                CUtensorMap* map)
 {
     const auto encode = tensor_map_encoder();
-    if (!encode || reinterpret_cast<uintptr_t>(vals) % 16 != 0) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)pair_entries(P.eg.Nv), (cuuint64_t)table_rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)pair_entries(P.eg.Nv) * pair_bytes};
+    if (!encode || reinterpret_cast<uintptr_t>(vals) % 16 != 0 || pitch * entry % 16 != 0) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)table_rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)(pitch * entry)};
     const cuuint32_t box[2] = {(cuuint32_t)S.rows, (cuuint32_t)S.cols}, step[2] = {1, 1};
-    return encode(map, pair_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_UINT32, 2,
-                  const_cast<void*>(vals), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUtensorMapDataType type = entry == 8   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
+                                     : entry == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32
+                                                  : CU_TENSOR_MAP_DATA_TYPE_UINT16;
+    return encode(map, type, 2, const_cast<void*>(vals), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -611,7 +454,7 @@ recon_status_t staged_quarter_gather(Plan& P, const ST* vals, size_t view_stride
     const unsigned view_rows = view_stride ? (unsigned)P.eg.Nu : 0u;
     const size_t table_rows = view_stride ? (size_t)P.eg.Nu * P.nviews : (size_t)P.eg.Nu;
     *served = table_rows < 0x7fffffff && staged_shape(P, slots, sizeof(ST), &S, &region, &smem) &&
-              pair_map(P, S, vals, 2 * sizeof(ST), table_rows, &map);
+              column_map(S, vals, pair_entries(P.eg.Nv), 2 * sizeof(ST), table_rows, &map);
     if (!*served) return RECON_OK;
     auto run = [&](auto ps) -> recon_status_t {
         constexpr int PS = decltype(ps)::value;

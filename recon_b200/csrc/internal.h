@@ -121,7 +121,10 @@ struct Plan {
     float* d_wq = nullptr;     // the same in the detector-column layout [u][v]
     float* d_colsino = nullptr;  // a sinogram in the detector-column layout (gather back projector input)
     unsigned colsino_views = 0;   // views d_colsino holds
-    bool bp_gather = false;    // Siddon back projection by the column gather (else ray-driven slabs)
+    bool bp_gather = false;    // Siddon back projection by the column gather (else the ray design)
+    bool bp_columns = false;   // the ray design along detector columns (else ray by ray in slabs)
+    unsigned* d_vmax = nullptr;  // bp_columns: max |value| (float bits) of the ratio's views [nviews], then of
+                                 // another input's [nviews + 1], then of the weights
     bool z_mirror = false;     // z table mirror-symmetric about z = 0: both projectors pair mirrored rows/voxels
     bool quarter = false;      // views n + N/4 a quarter turn from view n about a square volume, their xy
                                // tables exact rotations of view n's (the gather serves four columns a warp)
@@ -277,6 +280,12 @@ int exact_column_rows_default(const Plan& P, const std::vector<int4>& rect);
 std::string geometry_key(const Plan& P);
 void plan_release(Plan& P, void* p, size_t bytes);
 recon_status_t build_wq_pairs(Plan& P);
+recon_status_t build_view_maxima(Plan& P);
+void exact_use_gather(Plan& P, bool gather);
+size_t bp_acc_words(const Plan& P);
+template <class ST>
+recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, unsigned first, unsigned count,
+                          const unsigned* vmax, unsigned nmax, float* vol, const float* sens, cudaStream_t s);
 recon_status_t build_column_tiles(Plan& P, const std::vector<int4>& rect);
 recon_status_t exact_fp_column(Plan& P, const float* vol, unsigned first, unsigned count, float* out, cudaStream_t s);
 recon_status_t exact_fp_column_ratio(Plan& P, const float* vol, const void* g, void* ratio, int mode, int layout,

@@ -79,9 +79,8 @@ extern "C" recon_status_t recon_compat_bp_view_noalloc(const recon_geometry_t* g
     P.d_maxabs = reinterpret_cast<unsigned*>(scratch + 2);
     P.d_fix = scratch + kHeaderWords;
     cudaStream_t s = as_stream(stream);
-    // the accumulator must start at zero (the angle, loopN and maxabs slots
-    // are written or cleared by the projector itself)
-    RB_CUDA(cudaMemsetAsync(P.d_fix, 0, P.nvox * sizeof(unsigned long long), s));
+    // (the angle, loopN and maxabs slots and the accumulator are written or cleared by the
+    // projector itself)
     // view slot 0 (= P.nviews): angle and step count set up for this call
     return compat_bp_view(P, d_img, 0, true, angle_deg, d_vol, false, s);
 }
