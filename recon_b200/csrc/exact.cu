@@ -1123,7 +1123,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, PS <= 2 ? 3 : 2) bp_gather_
 // w (detector columns, wq) and the pairs along the pair index.
 template <class T>
 __global__ void __launch_bounds__(256) to_pairs_kernel(const T* __restrict__ in, const float* __restrict__ wq, int Nu,
-                                                        int Nv, T* __restrict__ out, unsigned* __restrict__ vmax)
+                                                        int Nv, T* __restrict__ out)
 {
     __shared__ float lo[32][33], hi[32][33];
     const int Np = Nv / 2 + 1;
@@ -1148,9 +1148,7 @@ __global__ void __launch_bounds__(256) to_pairs_kernel(const T* __restrict__ in,
         }
         const float wa = wq ? __ldg(wq + (size_t)u * Nv + p) : 1.0f;
         const float wb = wq ? __ldg(wq + (size_t)u * Nv + (Nv - 1 - p)) : 1.0f;
-        const float a = lo[threadIdx.x][threadIdx.y + 8 * q] * wa, b = hi[threadIdx.x][threadIdx.y + 8 * q] * wb;
-        store_pair<T>(o, a, b);
-        if (vmax) raise_max(vmax + blockIdx.z, max_bits(a, b));
+        store_pair<T>(o, lo[threadIdx.x][threadIdx.y + 8 * q] * wa, hi[threadIdx.x][threadIdx.y + 8 * q] * wb);
     }
 }
 
@@ -2216,14 +2214,14 @@ void exact_use_gather(Plan& P, bool gather)
     P.col_pairs = gather && exact_pairs_suit(P);
 }
 
-// Views of a sinogram [view][v][u] times w into the gather's input d_colsino; with vmax,
-// vmax[view] (zero before) their largest |value|.
+// Views of a sinogram [view][v][u] times w into the back projector's layout, d_colsino;
+// with vmax (detector columns), vmax[view] (zero before) their largest |value|.
 static recon_status_t to_gather_layout(Plan& P, const float* sino, unsigned count, unsigned* vmax, cudaStream_t s)
 {
     const ExactGeom& E = P.eg;
     if (!P.col_pairs) return to_columns<float>(P, sino, P.d_w, count, nullptr, P.d_colsino, s, vmax);
     exact::to_pairs_kernel<float><<<dim3((E.Nu + 31) / 32, (pair_entries(E.Nv) + 31) / 32, count), dim3(32, 8), 0, s>>>(
-        sino, P.d_wq, E.Nu, E.Nv, P.d_colsino, vmax);
+        sino, P.d_wq, E.Nu, E.Nv, P.d_colsino);
     RB_CUDA(cudaGetLastError());
     return RECON_OK;
 }

@@ -39,6 +39,7 @@
 namespace rb {
 namespace exact {
 
+constexpr int kWideBlocks = 8;  // blocks of kColRows threads per SM that the wide kernel's registers allow
 constexpr int kColRows = 128;  // at most this many detector rows per CTA (one warp per 32; the plan picks 32, 64 or 128)
 
 // Number of b in [0, n) whose plane value fmaf(q0 + b*d, S, O) lies before t
@@ -92,7 +93,9 @@ __device__ __forceinline__ void kahan_add(float& acc, float& comp, float x)
 // its next plane at infinity.  COUNT: no volume reads; the result is the
 // number of pieces of positive length the row has inside the volume (its
 // (ray, voxel) pairs).
-template <bool KAHAN, bool FAST, int STEP, bool COUNT>
+// WIDE: a block's pieces are found and their loads issued before any is summed (the same
+// sums; registers for eight pieces).
+template <bool KAHAN, bool FAST, int STEP, bool COUNT, bool WIDE>
 __device__ __forceinline__ float walk_rows(const float* __restrict__ volz, const float2* spc, int jb, int je, float cur,
                                            int kaddr, float kf, float tzn, float S, float O, int step, int kexit,
                                            int Z)
@@ -126,8 +129,36 @@ __device__ __forceinline__ float walk_rows(const float* __restrict__ volz, const
     int j = jb;
     for (; j + 7 <= je; j += 8) {
         float blk = 0.0f;
+        if constexpr (WIDE && !COUNT) {
+            float L0[8], L1[8], a0[8], a1[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) piece(j + q, blk);
+            for (int q = 0; q < 8; ++q) {
+                const float2 pc = spc[j + q];
+                const float* p = volz + (__float_as_int(pc.y) + kaddr);
+                const bool cross = tzn < pc.x;
+                const float m = fminf(tzn, pc.x);
+                L0[q] = m - cur;
+                L1[q] = pc.x - m;
+                a0[q] = __ldg(p);
+                a1[q] = 0.0f;
+                if (cross) {
+                    a1[q] = __ldg(p + st);
+                    kaddr += st;
+                    kf += fst;
+                    tzn = fmaf(kf, S, O);
+                    if (!FAST && kaddr == kexit) tzn = __int_as_float(0x7f800000);
+                }
+                cur = pc.x;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                blk = fmaf(L0[q], a0[q], blk);
+                blk = fmaf(L1[q], a1[q], blk);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) piece(j + q, blk);
+        }
         if (KAHAN && !COUNT) kahan_add(acc, comp, blk);
         else acc += blk;
     }
@@ -210,7 +241,7 @@ __device__ __forceinline__ RowWalk row_walk(const ExactGeom& G, const ZParam* __
 // f[voxel] (the projection divided by w), for the column path in spc (n pieces
 // from t_in to t_out), or with COUNT the row's number of (ray, voxel) pairs.
 // Called by whole warps.
-template <bool KAHAN, bool COUNT>
+template <bool KAHAN, bool COUNT, bool WIDE>
 __device__ __forceinline__ float column_row_sum(const ExactGeom& G, const ZParam* __restrict__ zp,
                                                 const float* __restrict__ volz, const float2* spc, int n, float t_in,
                                                 float t_out, int v, bool valid)
@@ -259,13 +290,13 @@ __device__ __forceinline__ float column_row_sum(const ExactGeom& G, const ZParam
     const bool up = __all_sync(0xffffffffu, !hit || dk > 0);
     const bool down = __all_sync(0xffffffffu, !hit || dk < 0);
     if (fast) {
-        if (up) return walk_rows<KAHAN, true, 1, COUNT>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
-        if (down) return walk_rows<KAHAN, true, -1, COUNT>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
-        return walk_rows<KAHAN, true, 0, COUNT>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
+        if (up) return walk_rows<KAHAN, true, 1, COUNT, WIDE>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
+        if (down) return walk_rows<KAHAN, true, -1, COUNT, WIDE>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
+        return walk_rows<KAHAN, true, 0, COUNT, WIDE>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
     }
-    if (up) return walk_rows<KAHAN, false, 1, COUNT>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
-    if (down) return walk_rows<KAHAN, false, -1, COUNT>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
-    return walk_rows<KAHAN, false, 0, COUNT>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
+    if (up) return walk_rows<KAHAN, false, 1, COUNT, WIDE>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
+    if (down) return walk_rows<KAHAN, false, -1, COUNT, WIDE>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
+    return walk_rows<KAHAN, false, 0, COUNT, WIDE>(volz, spc, jb, je, t_start, kaddr, kf, tzn, Z.S, Z.O, dk, kexit, G.Z);
 }
 
 // Rows mirrored about the source plane z = 0 (the plan's z table mirror-
@@ -275,7 +306,7 @@ __device__ __forceinline__ float column_row_sum(const ExactGeom& G, const ZParam
 // test and plane update, two loads and two sums.  The mirror's layer is
 // Z-1-k, at offset Z + 1 - kaddr of its padded column.  Returns {row v, row
 // Nv-1-v}.
-template <bool KAHAN, bool FAST, bool COUNT, bool PAIRED>
+template <bool KAHAN, bool FAST, bool COUNT, bool PAIRED, bool WIDE>
 __device__ __forceinline__ float2 walk_rows_mirror(const float* __restrict__ volz, const float2* spc, int jb, int je,
                                                    float cur, int kaddr, float kf, float tzn, float S, float O, int Z)
 {
@@ -325,7 +356,41 @@ __device__ __forceinline__ float2 walk_rows_mirror(const float* __restrict__ vol
     // the warp)
     for (; j + 15 <= je; j += 16) {
         float blk = 0.0f, blkm = 0.0f;
-        if (!PAIRED) {
+        if constexpr (WIDE && !COUNT) {
+#pragma unroll
+            for (int h = 0; h < 16; h += 8) {
+                float L0[8], L1[8], a0[8], a1[8], b0[8], b1[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const float2 pc = spc[j + h + q];
+                    const float* p = volz + (__float_as_int(pc.y) + kaddr);
+                    const bool cross = tzn < pc.x;
+                    const float m = fminf(tzn, pc.x);
+                    L0[q] = m - cur;
+                    L1[q] = pc.x - m;
+                    a0[q] = __ldg(p);
+                    b0[q] = __ldg(p + dm);
+                    a1[q] = b1[q] = 0.0f;
+                    if (cross) {
+                        a1[q] = __ldg(p - 1);
+                        b1[q] = __ldg(p + dm + 1);
+                        kaddr -= 1;
+                        dm += 2;
+                        kf -= 1.0f;
+                        tzn = fmaf(kf, S, O);
+                        if (!FAST && kaddr == 0) tzn = __int_as_float(0x7f800000);
+                    }
+                    cur = pc.x;
+                }
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    blk = fmaf(L0[q], a0[q], blk);
+                    blk = fmaf(L1[q], a1[q], blk);
+                    blkm = fmaf(L0[q], b0[q], blkm);
+                    blkm = fmaf(L1[q], b1[q], blkm);
+                }
+            }
+        } else if (!PAIRED) {
 #pragma unroll
             for (int q = 0; q < 16; ++q) piece(j + q, blk, blkm);
         } else if ((j & 1) == 0) {
@@ -419,7 +484,7 @@ __device__ __forceinline__ RowWalk mirror_walk(const ExactGeom& G, const ZParam*
 }
 
 // column_row_sum for lower row v (v < Nv/2) and its mirror Nv-1-v.
-template <bool KAHAN, bool COUNT, bool PAIRED>
+template <bool KAHAN, bool COUNT, bool PAIRED, bool WIDE>
 __device__ __forceinline__ float2 column_row_sum_mirror(const ExactGeom& G, const ZParam* __restrict__ zp,
                                                         const float* __restrict__ volz, const float2* spc, int n,
                                                         float t_in, float t_out, int v, bool valid)
@@ -427,9 +492,9 @@ __device__ __forceinline__ float2 column_row_sum_mirror(const ExactGeom& G, cons
     const RowWalk W = mirror_walk(G, zp, spc, n, t_in, t_out, v, valid);
     if (W.jb > W.je) return make_float2(0.0f, 0.0f);
     if (W.fast)
-        return walk_rows_mirror<KAHAN, true, COUNT, PAIRED>(volz, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S,
+        return walk_rows_mirror<KAHAN, true, COUNT, PAIRED, WIDE>(volz, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S,
                                                             W.O, G.Z);
-    return walk_rows_mirror<KAHAN, false, COUNT, PAIRED>(volz, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O,
+    return walk_rows_mirror<KAHAN, false, COUNT, PAIRED, WIDE>(volz, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O,
                                                          G.Z);
 }
 
@@ -497,10 +562,11 @@ __device__ __forceinline__ int column_path(float2* spc, const ExactGeom& G, cons
 // from the tile list {view, u | vstart << 16} (blockIdx.x indexes it) or,
 // without one, u = blockIdx.x, vstart = blockIdx.y * blockDim.x, view = view0 +
 // blockIdx.z.
-// With vmax, MODE 1 raises vmax[view] to the largest |value| it writes (float bits).
+// With vmax, MODE 1 in detector columns raises vmax[view] to the largest |value| it writes
+// (float bits).
 // MIRROR: rows come in mirrored pairs (see walk_rows_mirror); the CTA's rows
 // are lower rows (below Nv/2) and each lane also produces its mirror row.
-template <bool KAHAN, int MODE, int LAYOUT, class GT, class OT, bool MIRROR = false>
+template <bool KAHAN, int MODE, int LAYOUT, class GT, class OT, bool MIRROR, bool WIDE>
 __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out, unsigned* __restrict__ vmax)
 {
     // piece j: {t where it ends, offset of its (x, y) voxel column in volz (int bits)}
@@ -536,8 +602,8 @@ __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __
     if (n > 0) {
         // the table read in pairs for whole-volume walks; the xy blocks' shorter
         // walks measured faster reading it piece by piece
-        if (MIRROR) sum = column_row_sum_mirror<KAHAN, COUNTING, (MODE < 4)>(G, zp, volz, spc, n, t_in, t_out, v, valid);
-        else sum.x = column_row_sum<KAHAN, COUNTING>(G, zp, volz, spc, n, t_in, t_out, v, valid);
+        if (MIRROR) sum = column_row_sum_mirror<KAHAN, COUNTING, (MODE < 4), WIDE>(G, zp, volz, spc, n, t_in, t_out, v, valid);
+        else sum.x = column_row_sum<KAHAN, COUNTING, WIDE>(G, zp, volz, spc, n, t_in, t_out, v, valid);
     }
     if (COUNTING) {
         unsigned long long c = valid ? (unsigned long long)sum.x + (unsigned long long)sum.y : 0ull;
@@ -568,7 +634,6 @@ __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __
             OT* const o = out + ((size_t)(view - view0) * G.Nu + u) * Np * 2;
             const float a = value(v, sum.x), b = value(G.Nv - 1 - v, sum.y);
             store_pair<OT>(o + 2 * v, a, b);
-            if (MODE == 1 && vmax) raise_max(vmax + view, max_bits(as_stored<OT>(a), as_stored<OT>(b)));
             if (v == G.Nv / 2 - 1) store_pair<OT>(o + 2 * (v + 1), b, a);  // entry Nv/2: rows Nv/2, Nv/2 - 1
         } else {
             auto emit = [&](int row, float acc) {
@@ -589,18 +654,26 @@ __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __
 template <bool KAHAN, int MODE, int LAYOUT, class GT, class OT, bool MIRROR = false>
 __global__ void __launch_bounds__(kColRows, 16) fp_column_kernel(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out, unsigned* __restrict__ vmax)
 {
-    column_kernel_body<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>(G, txy, kxy, zp, wq, tiles, view0, blk, volz, g, out, vmax);
+    column_kernel_body<KAHAN, MODE, LAYOUT, GT, OT, MIRROR, false>(G, txy, kxy, zp, wq, tiles, view0, blk, volz, g, out, vmax);
 }
 template <bool KAHAN, int MODE, int LAYOUT, class GT, class OT, bool MIRROR = false>
 __global__ void __launch_bounds__(kColRows) fp_column_block_kernel(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out, unsigned* __restrict__ vmax)
 {
-    column_kernel_body<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>(G, txy, kxy, zp, wq, tiles, view0, blk, volz, g, out, vmax);
+    column_kernel_body<KAHAN, MODE, LAYOUT, GT, OT, MIRROR, false>(G, txy, kxy, zp, wq, tiles, view0, blk, volz, g, out, vmax);
+}
+// The whole-volume walks with the loads of eight pieces in flight per lane (64 registers),
+// for launches of few warps, which hide little of each other's load latency.
+template <bool KAHAN, int MODE, int LAYOUT, class GT, class OT, bool MIRROR = false>
+__global__ void __launch_bounds__(kColRows, kWideBlocks) fp_column_wide_kernel(ExactGeom G, const float4* __restrict__ txy, const int2* __restrict__ kxy, const ZParam* __restrict__ zp, const float* __restrict__ wq, const uint2* __restrict__ tiles, unsigned view0, int4 blk, const float* __restrict__ volz, const GT* __restrict__ g, OT* __restrict__ out, unsigned* __restrict__ vmax)
+{
+    column_kernel_body<KAHAN, MODE, LAYOUT, GT, OT, MIRROR, true>(G, txy, kxy, zp, wq, tiles, view0, blk, volz, g, out, vmax);
 }
 // the kernel of a MODE
-template <int MODE, bool KAHAN, int LAYOUT, class GT, class OT, bool MIRROR>
+template <int MODE, bool KAHAN, int LAYOUT, class GT, class OT, bool MIRROR, bool WIDE = false>
 constexpr auto fp_column_kernel_of()
 {
-    if constexpr (MODE >= 4) return fp_column_block_kernel<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>;
+    if constexpr (WIDE) return fp_column_wide_kernel<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>;
+    else if constexpr (MODE >= 4) return fp_column_block_kernel<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>;
     else return fp_column_kernel<KAHAN, MODE, LAYOUT, GT, OT, MIRROR>;
 }
 
@@ -746,7 +819,6 @@ __global__ void __launch_bounds__(256) bp_column_finish_kernel(ExactGeom G, cons
         }
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const int x = x0 + threadIdx.y + 8 * r, z = z0 + threadIdx.x;
             tile[threadIdx.y + 8 * r][threadIdx.x] =
                 nonfinite ? __int_as_float(0x7fffffff) : (float)((double)(long long)q[r] * unscale);
         }
@@ -884,8 +956,7 @@ __global__ void __launch_bounds__(256) column_finish_kernel(ExactGeom G, const f
 template <int MODE, class GT, class OT>
 __global__ void __launch_bounds__(256) column_finish_pairs_kernel(ExactGeom G, const float* __restrict__ acc,
                                                                   const float* __restrict__ wq,
-                                                                  const GT* __restrict__ g, OT* __restrict__ out,
-                                                                  unsigned* __restrict__ vmax)
+                                                                  const GT* __restrict__ g, OT* __restrict__ out)
 {
     __shared__ float lo[32][33], hi[32][33];
     const int Np = G.Nv / 2 + 1;  // pairs; a column holds pair_entries(Nv) entries
@@ -916,7 +987,6 @@ __global__ void __launch_bounds__(256) column_finish_pairs_kernel(ExactGeom G, c
         const float a = value(p, MODE ? lo[threadIdx.x][threadIdx.y + 8 * q] : 0.0f);
         const float b = value(G.Nv - 1 - p, MODE ? hi[threadIdx.x][threadIdx.y + 8 * q] : 0.0f);
         store_pair<OT>(out + (((size_t)blockIdx.z * G.Nu + u) * pair_entries(G.Nv) + p) * 2, a, b);
-        if (MODE == 1 && vmax) raise_max(vmax + blockIdx.z, max_bits(as_stored<OT>(a), as_stored<OT>(b)));
     }
 }
 
@@ -1088,10 +1158,19 @@ recon_status_t exact_to_zfast(const Plan& P, const float* vol, cudaStream_t s)
 // volume is copied to the z-fastest layout first.  For MODE 0 the pixels
 // outside the tiles are zeroed; the MLEM ratio buffers are zero there from
 // allocation on.
+// wide: the kernel for launches of few warps (compensated sums of MODES 0 .. 2).
 template <int MODE, int LAYOUT, class GT, class OT>
-static auto column_kernel(const Plan& P)
+static auto column_kernel(const Plan& P, bool wide = false)
 {
     const bool kahan = P.opt.sum == RECON_SUM_KAHAN;
+    if constexpr (MODE < 3) {
+        if (wide && kahan) {
+            if constexpr (LAYOUT == kLayoutPairs) return exact::fp_column_kernel_of<MODE, true, LAYOUT, GT, OT, true, true>();
+            else
+                return P.z_mirror ? exact::fp_column_kernel_of<MODE, true, LAYOUT, GT, OT, true, true>()
+                                  : exact::fp_column_kernel_of<MODE, true, LAYOUT, GT, OT, false, true>();
+        }
+    }
     if constexpr (LAYOUT == kLayoutPairs) {  // only from the mirror-paired walk
         return kahan ? exact::fp_column_kernel_of<MODE, true, LAYOUT, GT, OT, true>()
                      : exact::fp_column_kernel_of<MODE, false, LAYOUT, GT, OT, true>();
@@ -1154,8 +1233,7 @@ static recon_status_t launch_column_blocks(Plan& P, const float* vol, unsigned f
         }
     if constexpr (MODE != 3 && LAYOUT == kLayoutPairs) {
         const dim3 grid((E.Nu + 31) / 32, (E.Nv / 2 + 1 + 31) / 32, count);
-        exact::column_finish_pairs_kernel<MODE, GT, OT><<<grid, dim3(32, 8), 0, s>>>(E, acc, P.d_wq, g, out,
-                                                                                    ratio_max<MODE>(P, first));
+        exact::column_finish_pairs_kernel<MODE, GT, OT><<<grid, dim3(32, 8), 0, s>>>(E, acc, P.d_wq, g, out);
         RB_CUDA(cudaGetLastError());
     } else if constexpr (MODE != 3) {
         const dim3 grid((E.Nu + 31) / 32, (E.Nv + 31) / 32, count);
@@ -1195,7 +1273,12 @@ static recon_status_t launch_column(Plan& P, const float* vol, unsigned first, u
     }
     if (MODE != 3) RB_CHECK(exact_to_zfast(P, vol, s));
     const size_t smem = (size_t)(E.X + E.Y + 2) * sizeof(float2);
-    auto kernel = column_kernel<MODE, LAYOUT, GT, OT>(P);
+    // The wide kernel's 32 warps an SM against the other's 64: where the launch is at most
+    // 16 rounds of them, or a block is one warp (an SM holds 32 blocks).  Wide against not:
+    // 256^3 one view 104 against 156 us, 64 views 661 / 686, 360 views 3100 / 2960;
+    // 200 x 200 x 120, 32 views 133 / 180, 240 views 681 / 660; 64^3, 90 views 35 / 42.
+    const bool wide = P.col_rows == 32 || (double)grid.x * grid.y * grid.z * (P.col_rows / 32) <= 16.0 * 32.0 * P.sm_count;
+    auto kernel = column_kernel<MODE, LAYOUT, GT, OT>(P, wide);
     if (smem > 48 * 1024) RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<grid, P.col_rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, P.d_wq, tiles, first,
                                                make_int4(0, E.X, 0, E.Y), P.d_vol_z, g, out, ratio_max<MODE>(P, 0));
