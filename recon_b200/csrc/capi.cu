@@ -320,8 +320,8 @@ recon_status_t recon_plan_create(const recon_geometry_t* geom, const recon_optio
             if (!gather) exact_use_gather(*P, false);
             if (P->bp_columns) {
                 RB_CHECK(build_view_maxima(*P));
-                RB_CHECK(P->alloc(&P->d_bpacc, bp_acc_words(*P), "back projection accumulator"));
-                RB_CHECK(P->alloc(&P->d_bpmax, 4, "back projection scale"));  // a FixScale
+                RB_CHECK(P->alloc(&P->d_bpacc, bp_acc_words(*P) + 1, "back projection accumulator"));  // cleared in pairs
+                RB_CHECK(P->alloc(&P->d_bpmax, 1, "back projection max"));
             } else if (!gather) {  // the ray-driven back projector's slab accumulators
                 const size_t slab = (size_t)P->eg.X * P->eg.Y * bp_slab_depth(*P);
                 RB_CHECK(P->alloc(&P->d_bpacc, slab, "back projection accumulator"));

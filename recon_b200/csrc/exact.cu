@@ -76,13 +76,15 @@ __device__ __forceinline__ void axis_params(const GeomD& G, double p1, double dp
     kc = (int)k;
 }
 
-__global__ void xy_table_kernel(GeomD G, const float* __restrict__ angles, unsigned view0, unsigned nview,
+// Views view0 .. view0 + nview - 1, at angles[view] degrees or, without angles, all at
+// `angle`.
+__global__ void xy_table_kernel(GeomD G, const float* __restrict__ angles, float angle, unsigned view0, unsigned nview,
                                 float4* __restrict__ txy, int2* __restrict__ kxy, float2* __restrict__ cs)
 {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned view = view0 + blockIdx.y;
     if (u >= G.Nu || blockIdx.y >= nview) return;
-    const double th = (double)angles[view] / 180.0;
+    const double th = (double)(angles ? angles[view] : angle) / 180.0;
     const double c = cospi(th), s = sinpi(th);
     // detector x of column u after the misalignment shift/scale (no tilt):
     // calc_points12, siddon_device_kernelsMLEM.cuh:310-316
@@ -1170,12 +1172,10 @@ __global__ void wq_pairs_kernel(const float* __restrict__ wq, int Nu, int Nv, fl
 // layout [view][u][v] that the gather back projectors read: 32x32 (u, v) tiles
 // through shared memory, read and written along rows of 128 bytes.  With rect
 // (per view {u_min, u_max, v_min, v_max}), tiles wholly outside a view's
-// rectangle are skipped: the MLEM ratio is zero there in both layouts.  With vmax,
-// vmax[view] is raised to the largest |value| (float bits).
+// rectangle are skipped: the MLEM ratio is zero there in both layouts.
 template <class T>
 __global__ void __launch_bounds__(256) to_columns_kernel(const T* __restrict__ in, const float* __restrict__ w, int Nu,
-                                                         int Nv, const int4* __restrict__ rect, T* __restrict__ out,
-                                                         unsigned* __restrict__ vmax)
+                                                         int Nv, const int4* __restrict__ rect, T* __restrict__ out)
 {
     __shared__ T tile[32][33];
     const size_t view = blockIdx.z;
@@ -1186,14 +1186,12 @@ __global__ void __launch_bounds__(256) to_columns_kernel(const T* __restrict__ i
     }
     const T* __restrict__ src = in + view * Nu * Nv;
     T* __restrict__ dst = out + view * Nu * Nv;
-    float top = 0.0f;
     for (int r = threadIdx.y; r < 32; r += 8) {
         const int u = u0 + threadIdx.x, v = v0 + r;
         if (u < Nu && v < Nv) {
             T x = src[(size_t)v * Nu + u];
             if (w) x = T(float(x) * __ldg(w + (size_t)v * Nu + u));
             tile[r][threadIdx.x] = x;
-            top = max_bits(top, float(x));
         }
     }
     __syncthreads();
@@ -1201,7 +1199,6 @@ __global__ void __launch_bounds__(256) to_columns_kernel(const T* __restrict__ i
         const int v = v0 + threadIdx.x, u = u0 + r;
         if (u < Nu && v < Nv) dst[(size_t)u * Nv + v] = tile[threadIdx.x][r];
     }
-    if (vmax) raise_max(vmax + view, top);
 }
 
 // ---- back projection (ray-driven, into a z-slab) ---------------------------------------------
@@ -1359,7 +1356,7 @@ recon_status_t build_exact_tables(Plan& P, cudaStream_t s)
     P.quarter = quarter_turn_suits(P);
     if (P.nviews) {
         const unsigned direct = P.quarter ? P.nviews / 4 : P.nviews;  // views computed from their angles
-        exact::xy_table_kernel<<<dim3((G.Nu + 127) / 128, direct), 128, 0, s>>>(G, P.d_angles, 0u, direct, P.d_txy,
+        exact::xy_table_kernel<<<dim3((G.Nu + 127) / 128, direct), 128, 0, s>>>(G, P.d_angles, 0.0f, 0u, direct, P.d_txy,
                                                                               P.d_kxy, P.d_cs);
         RB_CUDA(cudaGetLastError());
         if (P.quarter) {
@@ -1375,13 +1372,10 @@ recon_status_t build_exact_tables(Plan& P, cudaStream_t s)
     return RECON_OK;
 }
 
-__global__ void exact_set_angle_kernel(float* p, float v) { *p = v; }
-
 recon_status_t exact_view_table(Plan& P, float angle, cudaStream_t s)
 {
     exact::GeomD G = geom_d(P);
-    exact_set_angle_kernel<<<1, 1, 0, s>>>(P.d_angles + P.nviews, angle);
-    exact::xy_table_kernel<<<dim3((G.Nu + 127) / 128, 1), 128, 0, s>>>(G, P.d_angles, P.nviews, 1u, P.d_txy,
+    exact::xy_table_kernel<<<dim3((G.Nu + 127) / 128, 1), 128, 0, s>>>(G, nullptr, angle, P.nviews, 1u, P.d_txy,
                                                                        P.d_kxy, P.d_cs);
     RB_CUDA(cudaGetLastError());
     return RECON_OK;
@@ -1576,12 +1570,12 @@ recon_status_t exact_fp(Plan& P, const float* vol, unsigned first, unsigned coun
 // (tiles outside them are left as they are), or null for every tile.
 template <class T>
 static recon_status_t to_columns(const Plan& P, const T* in, const float* w, unsigned count, const int4* rect, T* out,
-                                 cudaStream_t s, unsigned* vmax = nullptr)
+                                 cudaStream_t s)
 {
     for (unsigned v0 = 0; v0 < count; v0 += 65535) {
         const unsigned nv = std::min(count - v0, 65535u);
         exact::to_columns_kernel<T><<<dim3((P.eg.Nu + 31) / 32, (P.eg.Nv + 31) / 32, nv), dim3(32, 8), 0, s>>>(
-            in + (size_t)v0 * P.npix, w, P.eg.Nu, P.eg.Nv, rect ? rect + v0 : nullptr, out + (size_t)v0 * P.npix, vmax ? vmax + v0 : nullptr);
+            in + (size_t)v0 * P.npix, w, P.eg.Nu, P.eg.Nv, rect ? rect + v0 : nullptr, out + (size_t)v0 * P.npix);
         RB_CUDA(cudaGetLastError());
     }
     return RECON_OK;
@@ -1912,10 +1906,10 @@ recon_status_t exact_tune_bp(Plan& P)
     }
     exact_use_gather(P, gather);
     if (gather && P.d_bpacc) {
-        const size_t words = P.d_bpacc_t ? (size_t)P.eg.X * P.eg.Y * bp_slab_depth(P) : bp_acc_words(P);
+        const size_t words = P.d_bpacc_t ? (size_t)P.eg.X * P.eg.Y * bp_slab_depth(P) : bp_acc_words(P) + 1;
         plan_release(P, P.d_bpacc, words * sizeof(unsigned long long));
         plan_release(P, P.d_bpacc_t, words * sizeof(unsigned long long));
-        plan_release(P, P.d_bpmax, (P.d_bpacc_t ? 1 : 4) * sizeof(unsigned));
+        plan_release(P, P.d_bpmax, sizeof(unsigned));
         P.d_bpacc = P.d_bpacc_t = nullptr;
         P.d_bpmax = nullptr;
     }
@@ -2188,11 +2182,21 @@ recon_status_t build_wq_pairs(Plan& P)
 // The ray design's view maxima (bp_columns), the weights' among them.
 recon_status_t build_view_maxima(Plan& P)
 {
-    const size_t n = 2 * (size_t)P.nviews + 2;
+    const size_t n = (size_t)P.nviews + 1;
     RB_CHECK(P.alloc(&P.d_vmax, n, "view maxima"));
     RB_CUDA(cudaMemset(P.d_vmax, 0, n * sizeof(unsigned)));
     exact::maxabs_kernel<float><<<(unsigned)std::min<size_t>((P.npix + 255) / 256, (size_t)P.sm_count * 8), 256>>>(
         P.d_w, P.npix, nullptr, P.npix, P.d_vmax + n - 1);
+    RB_CUDA(cudaGetLastError());
+    return RECON_OK;
+}
+
+// *out = max(*out, the largest |value| times w of `count` views of a sinogram).
+recon_status_t launch_maxabs(Plan& P, const float* sino, unsigned count, unsigned* out, cudaStream_t s)
+{
+    const size_t n = (size_t)count * P.npix;
+    exact::maxabs_kernel<float><<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)P.sm_count * 8), 256, 0, s>>>(
+        sino, n, P.d_w, P.npix, out);
     RB_CUDA(cudaGetLastError());
     return RECON_OK;
 }
@@ -2214,12 +2218,11 @@ void exact_use_gather(Plan& P, bool gather)
     P.col_pairs = gather && exact_pairs_suit(P);
 }
 
-// Views of a sinogram [view][v][u] times w into the back projector's layout, d_colsino;
-// with vmax (detector columns), vmax[view] (zero before) their largest |value|.
-static recon_status_t to_gather_layout(Plan& P, const float* sino, unsigned count, unsigned* vmax, cudaStream_t s)
+// Views of a sinogram [view][v][u] times w into the gather's input d_colsino.
+static recon_status_t to_gather_layout(Plan& P, const float* sino, unsigned count, cudaStream_t s)
 {
     const ExactGeom& E = P.eg;
-    if (!P.col_pairs) return to_columns<float>(P, sino, P.d_w, count, nullptr, P.d_colsino, s, vmax);
+    if (!P.col_pairs) return to_columns<float>(P, sino, P.d_w, count, nullptr, P.d_colsino, s);
     exact::to_pairs_kernel<float><<<dim3((E.Nu + 31) / 32, (pair_entries(E.Nv) + 31) / 32, count), dim3(32, 8), 0, s>>>(
         sino, P.d_wq, E.Nu, E.Nv, P.d_colsino);
     RB_CUDA(cudaGetLastError());
@@ -2237,19 +2240,16 @@ recon_status_t exact_bp(Plan& P, const void* sino, bool sino_is_rw, bool bf16, u
     if (count == 0) return launch_fill(f_update ? f_update : vol, 0.0f, P.nvox, s);
     using bf = __nv_bfloat16;
     if (P.bp_columns) {
-        unsigned* const own = P.d_vmax + P.nviews;  // another input's views, then the weights
-        if (sens_mode) return bp_columns<float>(P, P.d_wq, 0, first, count, own + P.nviews + 1, 1u, vol, nullptr, s);
+        if (sens_mode) return bp_columns<float>(P, P.d_wq, 0, nullptr, first, count, P.d_vmax + P.nviews, 1u, vol, nullptr, s);
         float* const out = f_update ? f_update : vol;
         const float* const sn = f_update ? sens : nullptr;
         if (sino_is_rw) {  // the MLEM ratio of plan views
             const unsigned* m = P.d_vmax + first;
-            if (bf16) return bp_columns<bf>(P, (const bf*)sino, P.npix, first, count, m, count, out, sn, s);
-            return bp_columns<float>(P, (const float*)sino, P.npix, first, count, m, count, out, sn, s);
+            if (bf16) return bp_columns<bf>(P, (const bf*)sino, P.npix, nullptr, first, count, m, count, out, sn, s);
+            return bp_columns<float>(P, (const float*)sino, P.npix, nullptr, first, count, m, count, out, sn, s);
         }
-        RB_CHECK(ensure_column_scratch(P, count));
-        RB_CUDA(cudaMemsetAsync(own, 0, count * sizeof(unsigned), s));
-        RB_CHECK(to_gather_layout(P, (const float*)sino, count, own, s));
-        return bp_columns<float>(P, P.d_colsino, P.npix, first, count, own, count, vol, nullptr, s);
+        // a sinogram [view][v][u], read and weighted in place
+        return bp_columns<float>(P, (const float*)sino, P.npix, P.d_wq, first, count, nullptr, 0u, vol, nullptr, s);
     }
     if (P.bp_gather) {
         const size_t qv = column_view_elems(P);
@@ -2266,7 +2266,7 @@ recon_status_t exact_bp(Plan& P, const void* sino, bool sino_is_rw, bool bf16, u
         }
         // a sinogram [view][v][u]: weighted by w into the gather's layout first
         RB_CHECK(ensure_column_scratch(P, count));
-        RB_CHECK(to_gather_layout(P, (const float*)sino, count, nullptr, s));
+        RB_CHECK(to_gather_layout(P, (const float*)sino, count, s));
         return launch_gather<false, float>(P, P.d_colsino, qv, first, count, vol, nullptr, s);
     }
     if (sens_mode) return launch_bp<1, false, float>(P, nullptr, first, count, vol, nullptr, s);

@@ -116,12 +116,6 @@ __device__ __forceinline__ void raise_max(unsigned* slot, float value)
     asm("mov.u32 %0, %%laneid;" : "=r"(lane));
     if (bits && lane == (unsigned)__ffs(active) - 1u) atomicMax(slot, bits);
 }
-// The larger of two magnitudes as their float bits order them (NaN above infinity).
-__device__ __forceinline__ float max_bits(float a, float b)
-{
-    return __uint_as_float(max(__float_as_uint(fabsf(a)), __float_as_uint(fabsf(b))));
-}
-
 // ---- ray blocks ---------------------------------------------------------------------------
 
 // Rays are launched in blocks of 32 (u) x 4 (v).  A CTA's block comes from a

@@ -184,7 +184,7 @@ struct RowWalk {
 };
 
 __device__ __forceinline__ RowWalk row_walk(const ExactGeom& G, const ZParam* __restrict__ zp, const float2* spc, int n,
-                                            float t_in, float t_out, int v, bool valid)
+                                            float t_in, float t_out, int v, bool valid, int jlo, int jhi)
 {
     RowWalk W;
     ZParam Z;
@@ -203,8 +203,13 @@ __device__ __forceinline__ RowWalk row_walk(const ExactGeom& G, const ZParam* __
     W.jb = INT_MAX;
     W.je = -1;
     if (W.hit) {
-        W.jb = first_piece_ending<true>(spc, n, ta);
-        W.je = first_piece_ending<false>(spc, n, tb);
+        W.jb = max(first_piece_ending<true>(spc, n, ta), jlo);
+        W.je = min(first_piece_ending<false>(spc, n, tb), jhi);
+        if (W.jb > W.je) {  // none of its pieces are among these
+            W.hit = false;
+            W.jb = INT_MAX;
+            W.je = -1;
+        }
     }
     W.jb = __reduce_min_sync(0xffffffffu, W.jb);
     W.je = __reduce_max_sync(0xffffffffu, W.je);
@@ -432,7 +437,7 @@ __device__ __forceinline__ float2 walk_rows_mirror(const float* __restrict__ vol
 // row_walk for lower row v (v < Nv/2), which descends along t (S < 0: its next plane is
 // the layer's own), and its mirror Nv-1-v.
 __device__ __forceinline__ RowWalk mirror_walk(const ExactGeom& G, const ZParam* __restrict__ zp, const float2* spc, int n,
-                                               float t_in, float t_out, int v, bool valid)
+                                               float t_in, float t_out, int v, bool valid, int jlo, int jhi)
 {
     RowWalk W;
     ZParam Z;
@@ -452,8 +457,13 @@ __device__ __forceinline__ RowWalk mirror_walk(const ExactGeom& G, const ZParam*
     W.jb = INT_MAX;
     W.je = -1;
     if (W.hit) {
-        W.jb = first_piece_ending<true>(spc, n, ta);
-        W.je = first_piece_ending<false>(spc, n, tb);
+        W.jb = max(first_piece_ending<true>(spc, n, ta), jlo);
+        W.je = min(first_piece_ending<false>(spc, n, tb), jhi);
+        if (W.jb > W.je) {  // none of its pieces are among these
+            W.hit = false;
+            W.jb = INT_MAX;
+            W.je = -1;
+        }
     }
     W.jb = __reduce_min_sync(0xffffffffu, W.jb);
     W.je = __reduce_max_sync(0xffffffffu, W.je);
@@ -489,7 +499,7 @@ __device__ __forceinline__ float2 column_row_sum_mirror(const ExactGeom& G, cons
                                                         const float* __restrict__ volz, const float2* spc, int n,
                                                         float t_in, float t_out, int v, bool valid)
 {
-    const RowWalk W = mirror_walk(G, zp, spc, n, t_in, t_out, v, valid);
+    const RowWalk W = mirror_walk(G, zp, spc, n, t_in, t_out, v, valid, 0, INT_MAX);
     if (W.jb > W.je) return make_float2(0.0f, 0.0f);
     if (W.fast)
         return walk_rows_mirror<KAHAN, true, COUNT, PAIRED, WIDE>(volz, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S,
@@ -726,19 +736,23 @@ __device__ __forceinline__ void scatter_rows(unsigned long long* acc, const floa
     }
 }
 
-// Detector columns as the forward kernel takes them (tiles, or the full grid from row v0).
-// vals: values times w in detector columns [view - view0][u][v], or with view_stride 0
-// one table for every view.
+// Detector columns as the forward kernel takes them (tiles, or the full grid from row v0),
+// each path in nseg stretches, one per block (blockIdx.y of a tile, blockIdx.z % nseg).
+// vals: values times w in detector columns [view - view0][u][v], with view_stride 0 one table
+// for every view, or with wq a sinogram's values [view - view0][v][u], still to be weighted.
 template <bool MIRROR>
 __global__ void __launch_bounds__(kColRows) bp_column_kernel(ExactGeom G, const float4* __restrict__ txy,
                                                              const int2* __restrict__ kxy, const ZParam* __restrict__ zp,
                                                              const uint2* __restrict__ tiles, unsigned view0, int v0,
-                                                             const float* __restrict__ valsf,
+                                                             int nseg, const float* __restrict__ valsf,
                                                              const __nv_bfloat16* __restrict__ valsb, size_t view_stride,
-                                                             const FixScale* __restrict__ fix,
-                                                             unsigned long long* __restrict__ acc)
+                                                             const float* __restrict__ wq,
+                                                             const unsigned* __restrict__ maxabs, float max_len,
+                                                             int count_bits, unsigned long long* __restrict__ acc)
 {
     extern __shared__ float2 spc[];
+    __shared__ float scale_s;
+    if (threadIdx.x == 0) scale_s = fix_scale_of(__ldg(maxabs), max_len, count_bits).scale;
     unsigned view;
     int u, vstart;
     if (tiles) {
@@ -747,22 +761,21 @@ __global__ void __launch_bounds__(kColRows) bp_column_kernel(ExactGeom G, const 
         u = (int)(t.y & 0xffffu);
         vstart = (int)(t.y >> 16);
     } else {
-        view = view0 + blockIdx.z;
+        view = view0 + blockIdx.z / nseg;
         u = (int)blockIdx.x;
         vstart = v0 + (int)(blockIdx.y * blockDim.x);
     }
+    const int seg = (int)(tiles ? blockIdx.y : blockIdx.z % nseg);
     const int vend = MIRROR ? G.Nv / 2 : G.Nv;
     const int v = vstart + (int)threadIdx.x;
     const bool valid = v < vend;
     // the value(s) of the lane's row(s): every load before any is used
-    const size_t pc = (size_t)(view - view0) * view_stride + (size_t)u * G.Nv;
-    float x = 0.0f, xm = 0.0f;
-    if (valid) {
-        x = valsf ? __ldg(valsf + pc + v) : load_val<__nv_bfloat16>(valsb + pc + v);
-        if (MIRROR) xm = valsf ? __ldg(valsf + pc + (G.Nv - 1 - v)) : load_val<__nv_bfloat16>(valsb + pc + (G.Nv - 1 - v));
-    }
-    const float scale = __ldg(&fix->scale);
-    if (scale == 0.0f) return;  // the whole block: all zero or not finite
+    const size_t base = (size_t)(view - view0) * view_stride, pc = (size_t)u * G.Nv;
+    auto value = [&](int row) {
+        if (wq) return __ldg(valsf + base + (size_t)row * G.Nu + u) * __ldg(wq + pc + row);
+        return valsf ? __ldg(valsf + base + pc + row) : load_val<__nv_bfloat16>(valsb + base + pc + row);
+    };
+    const float x = valid ? value(v) : 0.0f, xm = (MIRROR && valid) ? value(G.Nv - 1 - v) : 0.0f;
     const float4 T = __ldg(txy + (size_t)view * G.Nu + u);
     const int2 K = __ldg(kxy + (size_t)view * G.Nu + u);
     const int4 b = make_int4(0, G.X, 0, G.Y);
@@ -772,10 +785,12 @@ __global__ void __launch_bounds__(kColRows) bp_column_kernel(ExactGeom G, const 
     const float t_out = fminf(fmaxf(x0, x1), fmaxf(y0, y1));
     const int n = column_path(spc, G, T, K, b, t_in, t_out);
     __syncthreads();
-    if (n == 0 || v - (int)(threadIdx.x & 31u) >= vend) return;  // whole warps
+    const float scale = scale_s;  // 0: all zero or not finite, nothing to add
+    if (n == 0 || scale == 0.0f || v - (int)(threadIdx.x & 31u) >= vend) return;  // whole warps
+    const int jlo = (int)((long long)n * seg / nseg), jhi = (int)((long long)n * (seg + 1) / nseg) - 1;
     const float cv = x * scale, cvm = xm * scale;
-    const RowWalk W = MIRROR ? mirror_walk(G, zp, spc, n, t_in, t_out, v, valid && (cv != 0.0f || cvm != 0.0f))
-                             : row_walk(G, zp, spc, n, t_in, t_out, v, valid && cv != 0.0f);
+    const RowWalk W = MIRROR ? mirror_walk(G, zp, spc, n, t_in, t_out, v, valid && (cv != 0.0f || cvm != 0.0f), jlo, jhi)
+                             : row_walk(G, zp, spc, n, t_in, t_out, v, valid && cv != 0.0f, jlo, jhi);
     if (W.jb > W.je) return;  // no row of the warp crosses the volume with a value
     const float a = W.hit ? cv : 0.0f, am = W.hit ? cvm : 0.0f;
     if (MIRROR) {
@@ -793,13 +808,17 @@ __global__ void __launch_bounds__(kColRows) bp_column_kernel(ExactGeom G, const 
 // against 41 us without and 28 us for a memset before the next sums.)  MODE 0: vol = Ht; MODE 2: the MLEM update, as
 // bp_finish_kernel (exact.cu).
 template <int MODE>
-__global__ void __launch_bounds__(256) bp_column_finish_kernel(ExactGeom G, const FixScale* __restrict__ fix,
+__global__ void __launch_bounds__(256) bp_column_finish_kernel(ExactGeom G, const unsigned* __restrict__ maxabs,
+                                                               float max_len, int count_bits,
                                                                const unsigned long long* __restrict__ acc,
                                                                float* __restrict__ vol, const float* __restrict__ sens)
 {
     __shared__ float tile[32][33];
-    const bool nonfinite = __ldg(&fix->nonfinite);  // a non-finite input value makes every voxel NaN
-    const double unscale = __ldg(&fix->unscale);
+    __shared__ FixScale fix;
+    if (threadIdx.x + threadIdx.y == 0) fix = fix_scale_of(__ldg(maxabs), max_len, count_bits);
+    __syncthreads();
+    const bool nonfinite = fix.nonfinite;  // a non-finite input value makes every voxel NaN
+    const double unscale = fix.unscale;
     const int tx = (G.X + 31) / 32, x0 = (int)(blockIdx.x % tx) * 32, z0 = (int)(blockIdx.x / tx) * 32;
     for (int y = blockIdx.y; y < G.Y; y += gridDim.y) {
         unsigned long long q[4];
@@ -835,19 +854,22 @@ __global__ void __launch_bounds__(256) bp_column_finish_kernel(ExactGeom G, cons
     }
 }
 
-// The call's scale from its views' maxima m[0 .. n).
-__global__ void fix_scale_kernel(const unsigned* __restrict__ m, unsigned n, float max_len, int count_bits,
-                                 FixScale* __restrict__ out)
+// Clears the accumulator, and *top = max of m[0 .. n) (0 for n = 0).
+__global__ void __launch_bounds__(256) bp_clear_kernel(ulonglong2* __restrict__ acc, size_t pairs,
+                                                       const unsigned* __restrict__ m, unsigned n, unsigned* __restrict__ top)
 {
-    __shared__ unsigned top;
-    if (threadIdx.x == 0) top = 0u;
+    for (size_t q = blockIdx.x * (size_t)256 + threadIdx.x; q < pairs; q += (size_t)gridDim.x * 256)
+        acc[q] = make_ulonglong2(0ull, 0ull);
+    if (blockIdx.x != 0) return;
+    __shared__ unsigned all;
+    if (threadIdx.x == 0) all = 0u;
     __syncthreads();
     unsigned v = 0u;
-    for (unsigned q = threadIdx.x; q < n; q += blockDim.x) v = max(v, m[q]);
+    for (unsigned q = threadIdx.x; q < n; q += 256) v = max(v, m[q]);
     v = __reduce_max_sync(0xffffffffu, v);
-    if ((threadIdx.x & 31u) == 0u) atomicMax(&top, v);
+    if ((threadIdx.x & 31u) == 0u) atomicMax(&all, v);
     __syncthreads();
-    if (threadIdx.x == 0) *out = fix_scale_of(top, max_len, count_bits);
+    if (threadIdx.x == 0) *top = all;
 }
 
 // f[z][y][x] -> volz[(y*X + x)*(Z + 2) + z + 1], 32 (x) x 32 (z) tiles of one y
@@ -1286,19 +1308,26 @@ static recon_status_t launch_column(Plan& P, const float* vol, unsigned first, u
     return RECON_OK;
 }
 
+constexpr int kStretch = 32;  // voxels of x + y a stretch, at least
+
 // The ray design's back projection along detector columns: views [first, first + count) of
-// table slots, vals their values times w in detector columns (view_stride 0: one table for
-// every view), vmax[0 .. nmax) the views' largest magnitudes; vol = Ht, or with sens the
-// MLEM update of vol.
+// table slots, vals as bp_column_kernel takes them, vmax[0 .. nmax) the views' largest
+// magnitudes (found here for a sinogram that is still to be weighted, wq); vol = Ht, or with
+// sens the MLEM update of vol.
 template <class ST>
-recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, unsigned first, unsigned count,
+recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, const float* wq, unsigned first, unsigned count,
                           const unsigned* vmax, unsigned nmax, float* vol, const float* sens, cudaStream_t s)
 {
     const ExactGeom& E = P.eg;
-    RB_CUDA(cudaMemsetAsync(P.d_bpacc, 0, bp_acc_words(P) * sizeof(unsigned long long), s));
-    exact::FixScale* const fix = reinterpret_cast<exact::FixScale*>(P.d_bpmax);
-    exact::fix_scale_kernel<<<1, 256, 0, s>>>(vmax, nmax, bp_max_len(P), bp_count_bits(P, count), fix);
+    const bool sino_max = wq != nullptr;
+    const float max_len = bp_max_len(P);
+    const int cbits = bp_count_bits(P, count);
+    const size_t pairs = (bp_acc_words(P) + 1) / 2;
+    const unsigned blocks = (unsigned)std::min<size_t>((pairs + 255) / 256, (size_t)P.sm_count * 16);
+    exact::bp_clear_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<ulonglong2*>(P.d_bpacc), pairs, sino_max ? nullptr : vmax,
+                                                  sino_max ? 0u : nmax, P.d_bpmax);
     RB_CUDA(cudaGetLastError());
+    if (sino_max) RB_CHECK(launch_maxabs(P, (const float*)vals, count, P.d_bpmax, s));
     const size_t smem = (size_t)(E.X + E.Y + 2) * sizeof(float2);
     auto kernel = P.z_mirror ? exact::bp_column_kernel<true> : exact::bp_column_kernel<false>;
     if (smem > 48 * 1024) RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1307,7 +1336,14 @@ recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, unsigned 
     if constexpr (std::is_same<ST, float>::value) vf = vals;
     else vb = vals;
     auto launch = [&](dim3 grid, int rows, const uint2* tiles, int v0) -> recon_status_t {
-        kernel<<<grid, rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, tiles, first, v0, vf, vb, view_stride, fix, P.d_bpacc);
+        // a launch of few warps takes the paths in stretches (the sums do not care)
+        const double warps = (double)grid.x * grid.y * grid.z * (rows / 32);
+        const double most = std::max(1, (E.X + E.Y) / kStretch);  // pieces enough to be worth finding the path
+        const int nseg = (int)std::min({8.0, most, std::max(1.0, 32.0 * P.sm_count / warps)});
+        if (tiles) grid.y *= nseg;
+        else grid.z *= nseg;
+        kernel<<<grid, rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, tiles, first, v0, nseg, vf, vb, view_stride, wq, P.d_bpmax,
+                                        max_len, cbits, P.d_bpacc);
         RB_CUDA(cudaGetLastError());
         return RECON_OK;
     };
@@ -1325,16 +1361,16 @@ recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, unsigned 
     }
     const dim3 fgrid((unsigned)((E.X + 31) / 32) * (unsigned)((E.Z + 31) / 32), std::min(E.Y, 65535));
     if (sens)
-        exact::bp_column_finish_kernel<2><<<fgrid, dim3(32, 8), 0, s>>>(E, fix, P.d_bpacc, vol, sens);
+        exact::bp_column_finish_kernel<2><<<fgrid, dim3(32, 8), 0, s>>>(E, P.d_bpmax, max_len, cbits, P.d_bpacc, vol, sens);
     else
-        exact::bp_column_finish_kernel<0><<<fgrid, dim3(32, 8), 0, s>>>(E, fix, P.d_bpacc, vol, sens);
+        exact::bp_column_finish_kernel<0><<<fgrid, dim3(32, 8), 0, s>>>(E, P.d_bpmax, max_len, cbits, P.d_bpacc, vol, sens);
     RB_CUDA(cudaGetLastError());
     return RECON_OK;
 }
-template recon_status_t bp_columns<float>(Plan&, const float*, size_t, unsigned, unsigned, const unsigned*, unsigned,
-                                          float*, const float*, cudaStream_t);
-template recon_status_t bp_columns<__nv_bfloat16>(Plan&, const __nv_bfloat16*, size_t, unsigned, unsigned, const unsigned*,
-                                                  unsigned, float*, const float*, cudaStream_t);
+template recon_status_t bp_columns<float>(Plan&, const float*, size_t, const float*, unsigned, unsigned,
+                                          const unsigned*, unsigned, float*, const float*, cudaStream_t);
+template recon_status_t bp_columns<__nv_bfloat16>(Plan&, const __nv_bfloat16*, size_t, const float*, unsigned,
+                                                  unsigned, const unsigned*, unsigned, float*, const float*, cudaStream_t);
 
 // (ray, voxel) pairs of positive length over all plan views, as the column
 // kernel assigns them (synchronous; no volume is read).

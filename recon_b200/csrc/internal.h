@@ -124,7 +124,7 @@ struct Plan {
     bool bp_gather = false;    // Siddon back projection by the column gather (else the ray design)
     bool bp_columns = false;   // the ray design along detector columns (else ray by ray in slabs)
     unsigned* d_vmax = nullptr;  // bp_columns: max |value| (float bits) of the ratio's views [nviews], then of
-                                 // another input's [nviews + 1], then of the weights
+                                 // the weights
     bool z_mirror = false;     // z table mirror-symmetric about z = 0: both projectors pair mirrored rows/voxels
     bool quarter = false;      // views n + N/4 a quarter turn from view n about a square volume, their xy
                                // tables exact rotations of view n's (the gather serves four columns a warp)
@@ -283,8 +283,9 @@ recon_status_t build_wq_pairs(Plan& P);
 recon_status_t build_view_maxima(Plan& P);
 void exact_use_gather(Plan& P, bool gather);
 size_t bp_acc_words(const Plan& P);
+recon_status_t launch_maxabs(Plan& P, const float* sino, unsigned count, unsigned* out, cudaStream_t s);
 template <class ST>
-recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, unsigned first, unsigned count,
+recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, const float* wq, unsigned first, unsigned count,
                           const unsigned* vmax, unsigned nmax, float* vol, const float* sens, cudaStream_t s);
 recon_status_t build_column_tiles(Plan& P, const std::vector<int4>& rect);
 recon_status_t exact_fp_column(Plan& P, const float* vol, unsigned first, unsigned count, float* out, cudaStream_t s);
