@@ -185,31 +185,37 @@ class Plan:
         v = self.nproj if views is None else views
         return torch.zeros((v, self.nv, self.nu), dtype=dtype or torch.float32, device=f"cuda:{self.options.device}")
 
+    def _empty(self, shape):
+        """An output that the call overwrites whole."""
+        import torch
+
+        return torch.empty(shape, dtype=torch.float32, device=f"cuda:{self.options.device}")
+
     # --- projectors ---
     def fp_view(self, vol, angle: float, out=None):
-        out = self.new_sinogram(1)[0] if out is None else out
+        out = self._empty((self.nv, self.nu)) if out is None else out
         check(lib().recon_fp_view(self._h, _ptr(vol), float(angle), _ptr(out), _stream()))
         return out
 
     def fp_views(self, vol, first: int = 0, count: int | None = None, out=None):
         count = self.nproj - first if count is None else count
-        out = self.new_sinogram(count) if out is None else out
+        out = self._empty((count, self.nv, self.nu)) if out is None else out
         check(lib().recon_fp_views(self._h, _ptr(vol), first, count, _ptr(out), _stream()))
         return out
 
     def bp_view(self, img, angle: float, out=None):
-        out = self.new_volume() if out is None else out
+        out = self._empty(self.shape_vol) if out is None else out
         check(lib().recon_bp_view(self._h, _ptr(img), float(angle), _ptr(out), _stream()))
         return out
 
     def bp_views(self, sino, first: int = 0, count: int | None = None, out=None):
         count = self.nproj - first if count is None else count
-        out = self.new_volume() if out is None else out
+        out = self._empty(self.shape_vol) if out is None else out
         check(lib().recon_bp_views(self._h, _ptr(sino), first, count, _ptr(out), _stream()))
         return out
 
     def sensitivity(self, out=None):
-        out = self.new_volume() if out is None else out
+        out = self._empty(self.shape_vol) if out is None else out
         check(lib().recon_sensitivity(self._h, _ptr(out), _stream()))
         return out
 

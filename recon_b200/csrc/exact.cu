@@ -2267,6 +2267,9 @@ recon_status_t exact_bp(Plan& P, const void* sino, bool sino_is_rw, bool bf16, u
         // a sinogram [view][v][u]: weighted by w into the gather's layout first
         RB_CHECK(ensure_column_scratch(P, count));
         RB_CHECK(to_gather_layout(P, (const float*)sino, count, s));
+        bool served = false;
+        RB_CHECK(few_views_gather(P, P.d_colsino, qv, first, count, vol, s, &served));
+        if (served) return RECON_OK;
         return launch_gather<false, float>(P, P.d_colsino, qv, first, count, vol, nullptr, s);
     }
     if (sens_mode) return launch_bp<1, false, float>(P, nullptr, first, count, vol, nullptr, s);

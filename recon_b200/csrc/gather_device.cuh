@@ -96,4 +96,8 @@ template <int EPI, class ST>
 recon_status_t staged_quarter_gather(Plan& P, const ST* vals, size_t view_stride, float* vol, const float* sens,
                                      cudaStream_t s, unsigned long long* npairs, bool set, unsigned m0, unsigned mc,
                                      bool* served);
+// gather_few.cu
+recon_status_t few_views_gather(Plan& P, const float* vals, size_t view_stride, unsigned first, unsigned count, float* vol,
+                                cudaStream_t s, bool* served);
+
 }  // namespace rb

@@ -325,6 +325,16 @@ static int staged_span(const Plan& P, double d, double rad)
     return (int)std::floor(d / dmin * std::sqrt(1.0 + tan * tan) * std::fabs((double)E.Ry / E.du) + 0.05) + 1;
 }
 
+// Most detector columns that one voxel column meets in a view, or 0 for a volume that comes
+// near the source (where a piece could lie behind it).
+int staged_wide(const Plan& P)
+{
+    const ExactGeom& E = P.eg;
+    const double vx = E.vox[0], vy = E.vox[1];
+    const double rad = std::hypot(0.5 * E.X * vx + 32 * vx, 0.5 * E.Y * vy + 4 * vy) * 1.001;
+    return rad < 0.9 * (double)E.Rf ? staged_span(P, std::hypot(vx, vy), rad) : 0;
+}
+
 // The boxes that tiles read in chunks of 32 * slots of Zs slices, of a detector whose
 // columns have entries 0 .. top (in multiples of `align` entries): S->wide, cols and rows.
 // False where no staged gather serves: a volume that comes near the source (a piece could
@@ -392,8 +402,6 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     }();
     return fn;
 }
-
-bool staged_maps_available() { return tensor_map_encoder() != nullptr; }
 
 // A table of `table_rows` detector columns of `pitch` entries (a row pair, or a value; an
 // entry is moved as one element of `entry` bytes), read in boxes of S.rows entries x S.cols

@@ -181,7 +181,7 @@ __device__ __forceinline__ bool staged_item(const ExactGeom& G, const GatherCons
 // barriers and the base's alignment.
 constexpr size_t kStagedSmem = 227 * 1024 - sizeof(exact::StagedItem) * 32 * exact::kStagedWarps - 1536;
 
-bool staged_maps_available();
+int staged_wide(const Plan& P);
 bool staged_boxes(const Plan& P, int slots, int Zs, int top, int align, exact::StagedShape* S);
 bool column_map(const exact::StagedShape& S, const void* vals, size_t pitch, size_t entry, size_t table_rows,
                 CUtensorMap* map);
