@@ -5,7 +5,8 @@
 // per-view launches add into the volume), and the MLEM update
 // f <- f * Ht / sens fused into the epilogue when requested.  One thread per
 // voxel in general; one thread per (x, y) column and z-chunk in GEOMETRIC mode
-// without detector tilt, where a column projects to one detector column.
+// without detector tilt, where a column projects to one detector column; one
+// warp per column for the MLEM iteration there.
 //
 // REFERENCE mode keeps backward_projection2's arithmetic and its flat-array
 // bilinear taps (a tap beyond the image end reads 0).  GEOMETRIC mode uses the
