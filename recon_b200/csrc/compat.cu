@@ -718,29 +718,33 @@ static bool pow2_voxels(const Plan& P)
 
 // Forward projections of plan views (or the scratch slot) from `first`.  From kZfastViews
 // views on they read a copy of the volume whose z runs fastest, so that a warp's detector
-// rows read neighbouring addresses; for fewer the copy costs more than it gives.  The
-// copy is the plan's: an event orders the calls that use it, so that calls on several
-// streams stay independent (within a stream capture the order is the capture's).
+// rows read neighbouring addresses; for fewer the copy costs more than it gives.  The copy
+// goes to `scratch`, which belongs to the caller's own work, or without it to the plan's
+// d_vol_z, which all calls on the plan share: an event orders those, so that calls on
+// several streams stay independent.  A captured call, whose replays no event of the plan
+// can order, reads the caller's volume instead.
 template <int MODE>
 static recon_status_t launch_compat_fp(Plan& P, unsigned first, unsigned count, const float* vol, const float* g,
-                                       float* out, unsigned* maxabs, cudaStream_t s)
+                                       float* out, unsigned* maxabs, float* scratch, cudaStream_t s)
 {
     if (count == 0) return RECON_OK;
-    const bool copy = count >= kZfastViews && P.d_vol_z;
-    bool ordered = false;
-    if (copy) {
+    float* copy = count >= kZfastViews ? scratch : nullptr;
+    const bool shared = count >= kZfastViews && !scratch && P.d_vol_z;
+    if (shared) {
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         RB_CUDA(cudaStreamIsCapturing(s, &capturing));
-        ordered = capturing == cudaStreamCaptureStatusNone && P.vol_z_free;
-        if (ordered) RB_CUDA(cudaStreamWaitEvent(s, P.vol_z_free, 0));
-        RB_CHECK(launch_zfast(vol, P.d_vol_z, P.cg.dims[0], P.cg.dims[1], P.cg.dims[2], 0, s));
+        if (capturing == cudaStreamCaptureStatusNone) {
+            copy = P.d_vol_z;
+            RB_CUDA(cudaStreamWaitEvent(s, P.vol_z_free, 0));
+        }
     }
+    if (copy) RB_CHECK(launch_zfast(vol, copy, P.cg.dims[0], P.cg.dims[1], P.cg.dims[2], 0, s));
     auto kernel = pow2_voxels(P) ? compat::fp_kernel<MODE, true> : compat::fp_kernel<MODE, false>;
     kernel<<<walk_grid(P, count), walk_block(), 0, s>>>(P.cg, P.d_angles, P.d_loopN, first,
-                                                        copy ? strides_z(P) : strides_x(P), copy ? P.d_vol_z : vol, g, out,
+                                                        copy ? strides_z(P) : strides_x(P), copy ? copy : vol, g, out,
                                                         maxabs);
     RB_CUDA(cudaGetLastError());
-    if (ordered) RB_CUDA(cudaEventRecord(P.vol_z_free, s));
+    if (copy && shared) RB_CUDA(cudaEventRecord(P.vol_z_free, s));
     return RECON_OK;
 }
 
@@ -873,7 +877,7 @@ recon_status_t compat_fp(Plan& P, const float* vol, unsigned first, unsigned cou
         first = P.nviews;
         count = 1;
     }
-    return launch_compat_fp<0>(P, first, count, vol, nullptr, out, nullptr, s);
+    return launch_compat_fp<0>(P, first, count, vol, nullptr, out, nullptr, nullptr, s);
 }
 
 // Back projection of one view, scaled by its own largest magnitude.
@@ -992,7 +996,7 @@ recon_status_t compat_mlem_iteration(Plan& P, const float* g, float* f, cudaStre
     if (P.nviews == 0) return RECON_OK;
     RB_CUDA(cudaMemsetAsync(P.d_maxabs, 0, (P.nviews + 2) * sizeof(unsigned), s));
     float* ratio = static_cast<float*>(P.d_ratio);
-    RB_CHECK(launch_compat_fp<1>(P, 0u, P.nviews, f, g, ratio, P.d_maxabs, s));
+    RB_CHECK(launch_compat_fp<1>(P, 0u, P.nviews, f, g, ratio, P.d_maxabs, P.d_ht, s));  // (Ht is written later)
     compat::max_views_kernel<<<1, 256, 0, s>>>(P.d_maxabs, P.nviews, P.d_maxabs + P.nviews + 1);
     RB_CUDA(cudaGetLastError());
     RB_CHECK(compat_bp_all(P, ratio, P.npix, P.d_ht, s));
@@ -1004,7 +1008,7 @@ recon_status_t compat_mlem_iteration(Plan& P, const float* g, float* f, cudaStre
 recon_status_t compat_fp_ratio_all(Plan& P, const float* vol, const float* g, float* ratio, cudaStream_t s)
 {
     RB_CUDA(cudaMemsetAsync(P.d_maxabs, 0, (P.nviews + 1) * sizeof(unsigned), s));
-    return launch_compat_fp<1>(P, 0u, P.nviews, vol, g, ratio, P.d_maxabs, s);
+    return launch_compat_fp<1>(P, 0u, P.nviews, vol, g, ratio, P.d_maxabs, P.d_ht, s);  // (no other use of Ht here)
 }
 
 // ---- parity entry points --------------------------------------------------------------

@@ -133,7 +133,7 @@ struct Plan {
     float* d_vol_z = nullptr;  // z-fastest copy of the projected volume with a zero layer at each end:
                                // voxel (x, y, z) at [(y*X + x)*(Z + 2) + z + 1] (column forward projector);
                                // COMPAT: without the layers, [(y*X + x)*Z + z]
-    cudaEvent_t vol_z_free = nullptr;  // COMPAT: the last use of d_vol_z
+    cudaEvent_t vol_z_free = nullptr;  // COMPAT: the last use of d_vol_z (by calls outside stream captures)
     // back projection: fixed-point accumulators of one z-slab, image layout
     // and xy-transposed, and the max |value| of the call's input (float bits)
     unsigned long long* d_bpacc = nullptr;
@@ -171,9 +171,9 @@ struct Plan {
     void* d_ratio = nullptr;      // ratio sinogram (float or bf16) [nviews][npix]
     void* d_ratio_rm = nullptr;   // EXACT gather plans: the ratio as the forward projector writes it,
                                   // [view][v][u], before its transpose into d_ratio
-    float* d_ht = nullptr;        // COMPAT: Ht accumulator [nvox]
+    float* d_ht = nullptr;        // COMPAT: Ht accumulator [nvox]; before it, the iteration's z-fastest image
     unsigned long long* d_fix = nullptr;  // COMPAT: fixed-point accumulator [nvox]
-    unsigned* d_maxabs = nullptr; // COMPAT: per-view max |value| bits [nviews+1]
+    unsigned* d_maxabs = nullptr; // COMPAT: max |value| bits per view, scratch slot, several views [nviews+2]
     float* d_view_img = nullptr;  // scratch image [npix]
     size_t device_bytes = 0;
     std::vector<void*> allocations;
