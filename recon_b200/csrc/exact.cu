@@ -1975,8 +1975,7 @@ static recon_status_t launch_gather_quarter(Plan& P, const ST* vals, size_t view
     const exact::GatherConst C = gather_const(P, vol, sens);
     const size_t smem = quarter_dynamic_smem<PS>(P);
     auto kernel = exact::bp_gather_quarter_kernel<EPI, ST, PS, SET>;
-    if (smem + kQuarterStaticSmem > 48 * 1024)
-        RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem + kQuarterStaticSmem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, 227 * 1024 - kQuarterStaticSmem));
     constexpr int tx = exact::kGatherTileX, ty = exact::kGatherWarps / exact::kGatherTileX;
     const int H = E.X / 2;  // base columns: the quadrant x, y < X/2
     const dim3 grid((H + tx - 1) / tx, (H + ty - 1) / ty);
@@ -2004,7 +2003,7 @@ static recon_status_t launch_gather_slots(Plan& P, const ST* vals, size_t view_s
     const size_t static_smem = sizeof(exact::GatherView) * 32 * exact::kGatherWarps +          // sview
                                sizeof(float) * exact::kGatherWarps * SLOTS * 32 * (MIRROR ? 2 : 1);  // sacc2
     if (smem + static_smem > 48 * 1024)
-        RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        RB_CHECK(allow_dynamic_smem(kernel, (size_t)exact_bp_gather_max_rows() * sizeof(float4)));
     constexpr int tx = exact::kGatherTileX, ty = exact::kGatherWarps / exact::kGatherTileX;
     const dim3 grid((E.X + tx - 1) / tx, (E.Y + ty - 1) / ty);
     kernel<<<grid, exact::kGatherWarps * 32, smem, s>>>(E, C, P.d_txy, P.d_kxy, P.d_cs, P.d_zp, first, count, vals,

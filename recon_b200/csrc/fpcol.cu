@@ -1016,6 +1016,8 @@ __global__ void __launch_bounds__(256) column_finish_pairs_kernel(ExactGeom G, c
 
 // ---- host side -----------------------------------------------------------------------------
 
+constexpr size_t kPathSmem = 200 * 1024;  // a detector column's path in shared memory, at most
+
 // The column kernel needs every piece of a detector column's path to span less
 // than a voxel of z (0.9 at most: the column diagonal times the steepest row's
 // dz/dt, z being dz_v * (t + Rf) / R along row v's ray), int offsets into the
@@ -1030,7 +1032,7 @@ bool exact_fp_column_suits(const Plan& P)
     const double needle = diag * slope / vz;
     const double padded = (double)E.X * E.Y * (E.Z + 2.0);
     return needle < 0.9 && padded < 2147483647.0 && E.Nu <= 65535 && E.Nv <= 65535 && E.Y <= 65535 &&
-           (size_t)(E.X + E.Y + 2) * sizeof(float2) <= 200 * 1024;
+           (size_t)(E.X + E.Y + 2) * sizeof(float2) <= kPathSmem;
 }
 
 // Side of the xy blocks the column projector walks one at a time (0: the
@@ -1237,7 +1239,7 @@ static recon_status_t launch_column_blocks(Plan& P, const float* vol, unsigned f
     constexpr int BMODE = MODE == 3 ? 5 : 4;
     using BOT = typename std::conditional<MODE == 3, OT, float>::type;
     auto kernel = column_kernel<BMODE, MODE == 3 ? LAYOUT : kLayoutColumns, float, BOT>(P);
-    if (smem > 48 * 1024) RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, kPathSmem));
     BOT* bout;
     if constexpr (MODE == 3) bout = out;
     else bout = acc;
@@ -1301,7 +1303,7 @@ static recon_status_t launch_column(Plan& P, const float* vol, unsigned first, u
     // 200 x 200 x 120, 32 views 133 / 180, 240 views 681 / 660; 64^3, 90 views 35 / 42.
     const bool wide = P.col_rows == 32 || (double)grid.x * grid.y * grid.z * (P.col_rows / 32) <= 16.0 * 32.0 * P.sm_count;
     auto kernel = column_kernel<MODE, LAYOUT, GT, OT>(P, wide);
-    if (smem > 48 * 1024) RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, kPathSmem));
     kernel<<<grid, P.col_rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, P.d_wq, tiles, first,
                                                make_int4(0, E.X, 0, E.Y), P.d_vol_z, g, out, ratio_max<MODE>(P, 0));
     RB_CUDA(cudaGetLastError());
@@ -1330,7 +1332,7 @@ recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, const flo
     if (sino_max) RB_CHECK(launch_maxabs(P, (const float*)vals, count, P.d_bpmax, s));
     const size_t smem = (size_t)(E.X + E.Y + 2) * sizeof(float2);
     auto kernel = P.z_mirror ? exact::bp_column_kernel<true> : exact::bp_column_kernel<false>;
-    if (smem > 48 * 1024) RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, kPathSmem));
     const float* vf = nullptr;
     const __nv_bfloat16* vb = nullptr;
     if constexpr (std::is_same<ST, float>::value) vf = vals;

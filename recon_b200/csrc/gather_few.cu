@@ -145,6 +145,8 @@ __global__ void __launch_bounds__(kFewWarps * 32, 4) bp_gather_few_kernel(
 
 // ---- host side -----------------------------------------------------------------------------
 
+constexpr size_t kFewSmem = 64 * 1024;  // dynamic shared memory of the few-view kernel, at most
+
 static size_t few_smem(const Plan& P, unsigned count, int wide)
 {
     const size_t sets = (size_t)count * wide;
@@ -161,7 +163,7 @@ static int few_views_suit(const Plan& P, unsigned count)
 {
     if (!P.col_pairs || count == 0 || count > 4 || (count > 2 && (size_t)P.eg.X * P.eg.Y < 16384)) return 0;
     const int wide = staged_wide(P);
-    return wide > 0 && wide <= 4 && few_smem(P, count, wide) <= 64 * 1024 ? wide : 0;
+    return wide > 0 && wide <= 4 && few_smem(P, count, wide) <= kFewSmem ? wide : 0;
 }
 
 // Back projection of table slots first .. first + count - 1 from mirrored row pairs;
@@ -177,7 +179,7 @@ recon_status_t few_views_gather(Plan& P, const float* vals, size_t view_stride, 
     const dim3 grid((E.X + exact::kFewStage - 1) / exact::kFewStage, (E.Y + exact::kFewWarps - 1) / exact::kFewWarps);
     auto run = [&](auto ps) -> recon_status_t {
         auto kernel = exact::bp_gather_few_kernel<decltype(ps)::value>;
-        RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        RB_CHECK(allow_dynamic_smem(kernel, kFewSmem));
         kernel<<<grid, exact::kFewWarps * 32, smem, s>>>(E, gather_const(P, vol, nullptr), wide, P.d_txy, P.d_kxy, P.d_cs,
                                                          P.d_zp, first, (int)count, vals, view_stride, vol);
         RB_CUDA(cudaGetLastError());

@@ -29,6 +29,17 @@ recon_status_t cuda_fail(cudaError_t e, const char* what);
         if (rb_s_ != RECON_OK) return rb_s_;             \
     } while (0)
 
+// Lets `kernel` be launched with up to `most` bytes of dynamic shared memory.  The limit is
+// one value per kernel and device, which every thread's plans share, so a kernel is always
+// given the same one: with each launch's own size, another thread's smaller one between the
+// call and the launch made the launch fail (0.3 % of the launches of two threads).
+template <class Kernel>
+recon_status_t allow_dynamic_smem(Kernel kernel, size_t most)
+{
+    RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    return RECON_OK;
+}
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // ---- geometry passed to kernels by value ----------------------------------
