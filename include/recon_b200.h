@@ -393,6 +393,12 @@ recon_status_t recon_count_intersections(recon_plan_t plan, unsigned long long* 
 #define RECON_PROJECTOR_BACK 1
 recon_status_t recon_count_projector_pairs(recon_plan_t plan, int projector, unsigned long long* count);
 
+/* The kernel that the calling thread's last forward (RECON_PROJECTOR_FORWARD) or back
+ * projection (RECON_PROJECTOR_BACK) launched, of an MLEM iteration too: its name in the
+ * library's sources, "" before the first one, NULL for another projector.  A diagnostic:
+ * several kernels serve a call, by its sizes, with the same results. */
+const char* recon_last_kernel(int projector);
+
 /* ---- elementwise drop-ins (hf_cuda_kernels.cuh) -------------------------- */
 
 /* set_ones (hf_cuda_kernels.cuh:25-35) */

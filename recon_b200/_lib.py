@@ -127,6 +127,7 @@ def lib() -> C.CDLL:
         "recon_mlem_backward_update": (st, [P, P, P]),
         "recon_count_intersections": (st, [P, C.POINTER(C.c_ulonglong)]),
         "recon_count_projector_pairs": (st, [P, C.c_int, C.POINTER(C.c_ulonglong)]),
+        "recon_last_kernel": (C.c_char_p, [C.c_int]),
         "recon_view_step_count": (st, [P, f, up]),
         "recon_set_ones": (st, [P, C.c_size_t, P]),
         "recon_divide1": (st, [P, P, C.c_size_t, P]),
@@ -163,7 +164,7 @@ def exported_symbols() -> list[str]:
         "recon_add", "recon_compat_setup_view", "recon_compat_trace", "recon_view_step_count", "recon_mlem_from_cfg",
         "recon_forward_projection_from_cfg", "recon_backward_projection_from_cfg", "recon_batch_create",
         "recon_batch_destroy", "recon_batch_mlem", "recon_compat_bp_view_noalloc", "recon_osem",
-        "recon_upload_sinogram",
+        "recon_upload_sinogram", "recon_last_kernel",
     ]
 
 

@@ -304,6 +304,12 @@ class Plan:
         check(lib().recon_count_projector_pairs(self._h, int(projector), C.byref(n)))
         return int(n.value)
 
+    @staticmethod
+    def last_kernel(projector: int) -> str:
+        """The kernel that this thread's last PROJECTOR_FORWARD or PROJECTOR_BACK
+        projection launched (recon_last_kernel)."""
+        return lib().recon_last_kernel(int(projector)).decode()
+
     # --- parity (COMPAT) ---
     def compat_setup_view(self, angle: float) -> tuple[int, dict]:
         n = self.nu * self.nv

@@ -12,6 +12,9 @@ namespace rb {
 
 static thread_local std::string g_last_error;
 
+static thread_local const char* g_last_kernel[2] = {"", ""};  // by RECON_PROJECTOR_*
+
+void note_kernel(int projector, const char* name) { g_last_kernel[projector] = name; }
 void set_error(const std::string& msg) { g_last_error = msg; }
 recon_status_t fail(recon_status_t code, const std::string& msg)
 {
@@ -687,6 +690,11 @@ recon_status_t recon_count_projector_pairs(recon_plan_t P, int projector, unsign
     if (P->fp_column && (projector == RECON_PROJECTOR_FORWARD || P->bp_columns)) return exact_fp_column_count(*P, count);
     if (projector == RECON_PROJECTOR_BACK && P->bp_gather) return exact_bp_gather_count(*P, count);
     return exact_count(*P, count);  // the ray walk, which these projectors run
+}
+
+const char* recon_last_kernel(int projector)
+{
+    return projector == RECON_PROJECTOR_FORWARD || projector == RECON_PROJECTOR_BACK ? g_last_kernel[projector] : nullptr;
 }
 
 recon_status_t recon_mlem(recon_plan_t P, const void* d_g, unsigned iters, float* d_f, int init_ones, void* stream)

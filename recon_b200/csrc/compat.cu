@@ -740,6 +740,7 @@ static recon_status_t launch_compat_fp(Plan& P, unsigned first, unsigned count, 
     }
     if (copy) RB_CHECK(launch_zfast(vol, copy, P.cg.dims[0], P.cg.dims[1], P.cg.dims[2], 0, s));
     auto kernel = pow2_voxels(P) ? compat::fp_kernel<MODE, true> : compat::fp_kernel<MODE, false>;
+    note_kernel(RECON_PROJECTOR_FORWARD, "compat::fp_kernel");
     kernel<<<walk_grid(P, count), walk_block(), 0, s>>>(P.cg, P.d_angles, P.d_loopN, first,
                                                         copy ? strides_z(P) : strides_x(P), copy ? copy : vol, g, out,
                                                         maxabs);
@@ -772,6 +773,7 @@ static recon_status_t launch_scatter(Plan& P, unsigned first, unsigned views, co
     const bool pow2 = pow2_voxels(P);
     auto kernel = bands ? (pow2 ? compat::bp_scatter_kernel<true, true> : compat::bp_scatter_kernel<false, true>)
                         : (pow2 ? compat::bp_scatter_kernel<true, false> : compat::bp_scatter_kernel<false, false>);
+    note_kernel(RECON_PROJECTOR_BACK, "compat::bp_scatter_kernel");
     kernel<<<walk_grid(P, views), walk_block(), 0, s>>>(P.cg, P.d_angles, P.d_loopN, first, strides_z(P), img, img_stride,
                                                         P.d_maxabs, slot, R, P.d_fix);
     RB_CUDA(cudaGetLastError());

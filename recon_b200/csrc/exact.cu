@@ -1544,6 +1544,7 @@ static recon_status_t launch_fp(Plan& P, const float* vol, unsigned first, unsig
     ray_launch(P, P.fp_tiles, first, count, &grid, &tiles, &n_launch);
     if (tiles && MODE != 1 && MODE != 3 && MODE != 4) RB_CUDA(cudaMemsetAsync(out, 0, (size_t)count * P.npix * sizeof(OT), s));
     if (n_launch == 0) return RECON_OK;
+    note_kernel(RECON_PROJECTOR_FORWARD, "fp_kernel");
     RB_CHECK(exact_transpose(vol, P.d_vol_t, P.eg.X, P.eg.Y, P.eg.Z, s));
     const dim3 blk = fp_block();
     if (P.opt.sum == RECON_SUM_KAHAN)
@@ -1763,6 +1764,7 @@ static recon_status_t launch_bp(Plan& P, const ST* sino, unsigned first, unsigne
     const dim3 blk = fp_block();
     constexpr int RMODE = (MODE == 1) ? 1 : 0;
     const RayTiles none;
+    note_kernel(RECON_PROJECTOR_BACK, "bp_ray_kernel");
     for (int k0 = 0, slab = 0; k0 < P.eg.Z; k0 += depth, ++slab) {
         const int k1 = std::min(k0 + depth, P.eg.Z);
         dim3 grid;
@@ -1975,6 +1977,7 @@ static recon_status_t launch_gather_quarter(Plan& P, const ST* vals, size_t view
     const exact::GatherConst C = gather_const(P, vol, sens);
     const size_t smem = quarter_dynamic_smem<PS>(P);
     auto kernel = exact::bp_gather_quarter_kernel<EPI, ST, PS, SET>;
+    note_kernel(RECON_PROJECTOR_BACK, "bp_gather_quarter_kernel");
     if (smem + kQuarterStaticSmem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, 227 * 1024 - kQuarterStaticSmem));
     constexpr int tx = exact::kGatherTileX, ty = exact::kGatherWarps / exact::kGatherTileX;
     const int H = E.X / 2;  // base columns: the quadrant x, y < X/2
@@ -2002,6 +2005,8 @@ static recon_status_t launch_gather_slots(Plan& P, const ST* vals, size_t view_s
     }();
     const size_t static_smem = sizeof(exact::GatherView) * 32 * exact::kGatherWarps +          // sview
                                sizeof(float) * exact::kGatherWarps * SLOTS * 32 * (MIRROR ? 2 : 1);  // sacc2
+    note_kernel(RECON_PROJECTOR_BACK,
+                !MIRROR ? "bp_gather_kernel" : P.col_pairs ? "bp_gather_pairs_kernel" : "bp_gather_mirror_kernel");
     if (smem + static_smem > 48 * 1024)
         RB_CHECK(allow_dynamic_smem(kernel, (size_t)exact_bp_gather_max_rows() * sizeof(float4)));
     constexpr int tx = exact::kGatherTileX, ty = exact::kGatherWarps / exact::kGatherTileX;

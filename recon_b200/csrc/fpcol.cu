@@ -1225,6 +1225,7 @@ static recon_status_t launch_column_blocks(Plan& P, const float* vol, unsigned f
     const ExactGeom& E = P.eg;
     const size_t smem = (size_t)(E.X + E.Y + 2) * sizeof(float2);
     constexpr bool in_place = LAYOUT == kLayoutColumns && std::is_same<OT, float>::value;
+    note_kernel(RECON_PROJECTOR_FORWARD, "fp_column_block_kernel");
     float* acc = nullptr;
     if (MODE != 3) {
         if (in_place) {
@@ -1303,6 +1304,7 @@ static recon_status_t launch_column(Plan& P, const float* vol, unsigned first, u
     // 200 x 200 x 120, 32 views 133 / 180, 240 views 681 / 660; 64^3, 90 views 35 / 42.
     const bool wide = P.col_rows == 32 || (double)grid.x * grid.y * grid.z * (P.col_rows / 32) <= 16.0 * 32.0 * P.sm_count;
     auto kernel = column_kernel<MODE, LAYOUT, GT, OT>(P, wide);
+    note_kernel(RECON_PROJECTOR_FORWARD, wide && P.opt.sum == RECON_SUM_KAHAN && MODE < 3 ? "fp_column_wide_kernel" : "fp_column_kernel");
     if (smem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, kPathSmem));
     kernel<<<grid, P.col_rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, P.d_wq, tiles, first,
                                                make_int4(0, E.X, 0, E.Y), P.d_vol_z, g, out, ratio_max<MODE>(P, 0));
@@ -1332,6 +1334,7 @@ recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, const flo
     if (sino_max) RB_CHECK(launch_maxabs(P, (const float*)vals, count, P.d_bpmax, s));
     const size_t smem = (size_t)(E.X + E.Y + 2) * sizeof(float2);
     auto kernel = P.z_mirror ? exact::bp_column_kernel<true> : exact::bp_column_kernel<false>;
+    note_kernel(RECON_PROJECTOR_BACK, "bp_column_kernel");
     if (smem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, kPathSmem));
     const float* vf = nullptr;
     const __nv_bfloat16* vb = nullptr;

@@ -180,6 +180,7 @@ recon_status_t few_views_gather(Plan& P, const float* vals, size_t view_stride, 
     auto run = [&](auto ps) -> recon_status_t {
         auto kernel = exact::bp_gather_few_kernel<decltype(ps)::value>;
         RB_CHECK(allow_dynamic_smem(kernel, kFewSmem));
+        note_kernel(RECON_PROJECTOR_BACK, "bp_gather_few_kernel");
         kernel<<<grid, exact::kFewWarps * 32, smem, s>>>(E, gather_const(P, vol, nullptr), wide, P.d_txy, P.d_kxy, P.d_cs,
                                                          P.d_zp, first, (int)count, vals, view_stride, vol);
         RB_CUDA(cudaGetLastError());

@@ -430,6 +430,7 @@ static recon_status_t launch_staged(Plan& P, const exact::StagedShape& S, size_t
     const ExactGeom& E = P.eg;
     auto kernel = exact::bp_staged_quarter_kernel<EPI, ST, PS, RB, SET>;
     RB_CHECK(allow_dynamic_smem(kernel, 128 + kStagedSmem));
+    note_kernel(RECON_PROJECTOR_BACK, "bp_staged_quarter_kernel");
     const int H = E.X / 2;
     const dim3 grid((H + exact::kStagedTX - 1) / exact::kStagedTX, (H + exact::kStagedTY - 1) / exact::kStagedTY);
     kernel<<<grid, exact::kStagedThreads, smem, s>>>(E, gather_const(P, vol, sens), S, P.d_txy, P.d_kxy, P.d_cs, P.d_zp,

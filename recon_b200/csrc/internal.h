@@ -17,6 +17,8 @@ namespace rb {
 void set_error(const std::string& msg);
 recon_status_t fail(recon_status_t code, const std::string& msg);
 recon_status_t cuda_fail(cudaError_t e, const char* what);
+// The kernel that a projection of this thread launched (recon_last_kernel).
+void note_kernel(int projector, const char* name);
 
 #define RB_CUDA(call)                                            \
     do {                                                         \

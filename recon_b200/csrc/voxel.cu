@@ -679,6 +679,7 @@ static recon_status_t launch_voxel(Plan& P, const float* sino, const float* angl
             const int groups = staged_voxel_rows(G), slots = gather_slots(G.Z);
             const int taken = std::max(groups, slots);  // the instance's; all but its last group lie inside the image
             if (groups > 0 && taken <= slots + 1 && 32 * (taken - 1) <= G.Nv) {
+                note_kernel(RECON_PROJECTOR_BACK, "voxel::bp_staged_kernel");
                 switch (2 * slots + (taken > slots)) {
 #define RB_STAGED_SLOTS(n)                                                                                          \
     case 2 * n:                                                                                                     \
@@ -703,6 +704,7 @@ static recon_status_t launch_voxel(Plan& P, const float* sino, const float* angl
                 return RECON_OK;
             }
         }
+        note_kernel(RECON_PROJECTOR_BACK, "voxel::bp_gather_kernel");
         switch (gather_slots(G.Z)) {
 #define RB_VOXEL_SLOTS(n)                                                                                          \
     case n:                                                                                                        \
@@ -722,6 +724,8 @@ static recon_status_t launch_voxel(Plan& P, const float* sino, const float* angl
         RB_CUDA(cudaGetLastError());
         return RECON_OK;
     }
+    note_kernel(RECON_PROJECTOR_BACK,
+                VMODE == RECON_VOXEL_GEOMETRIC && untilted ? "voxel::bp_column_kernel" : "voxel::bp_kernel");
     if (VMODE == RECON_VOXEL_GEOMETRIC && untilted) {
         constexpr int ZC = 16;
         const dim3 cgrid((G.X + 31) / 32, (G.Y + 3) / 4, (G.Z + ZC - 1) / ZC);

@@ -1,0 +1,110 @@
+"""Which kernel serves a call: the geometries of the kernels' own tests take the kernels that
+they are there for, and the calls outside a kernel's bounds the one that it falls back to."""
+import pytest
+
+from conftest import small_cfg
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("no CUDA device", allow_module_level=True)
+
+from recon_b200 import (ARITH_COMPAT, BP_VOXEL, PROJECTOR_BACK, PROJECTOR_FORWARD, SIDDON_BP_GATHER,  # noqa: E402
+                        SIDDON_BP_RAY, SUM_PLAIN, Options, Plan)
+from test_gpu_few_views import GEOMS as FEW  # noqa: E402
+from test_gpu_fp_wide import BIG  # noqa: E402
+from test_gpu_ray_columns import GEOMS as RAY  # noqa: E402
+from test_gpu_staged import QUARTER  # noqa: E402
+from test_gpu_voxel_staged import GEOMS as VOXEL  # noqa: E402
+
+
+def back(P, count=None, first=0):
+    count = P.nproj - first if count is None else count
+    P.bp_views(torch.ones((count, P.nv, P.nu), device="cuda"), first, count)
+    return P.last_kernel(PROJECTOR_BACK)
+
+
+def forward(P, count=None):
+    P.fp_views(torch.ones(P.shape_vol, device="cuda"), 0, P.nproj if count is None else count)
+    return P.last_kernel(PROJECTOR_FORWARD)
+
+
+def iteration(P):
+    P.mlem_prepare()
+    P.mlem_iteration(P.new_sinogram(), P.new_volume(1.0))
+    return P.last_kernel(PROJECTOR_FORWARD), P.last_kernel(PROJECTOR_BACK)
+
+
+@pytest.mark.parametrize("name", list(QUARTER))
+def test_quarter_turns(name):
+    P = Plan(QUARTER[name], Options(siddon_bp=SIDDON_BP_GATHER))
+    assert back(P) == "bp_staged_quarter_kernel"
+    assert iteration(P)[1] == "bp_staged_quarter_kernel"
+    assert back(P, 3) != "bp_staged_quarter_kernel"
+    P.mlem_forward_quarters(P.new_sinogram(), P.new_volume(1.0), 0, 1)
+    P.mlem_backward_quarters(P.new_volume(), 0, 1)
+    assert P.last_kernel(PROJECTOR_BACK) == "bp_staged_quarter_kernel"
+
+
+def test_quarter_turns_without_stages():
+    """More rows than a box holds; a box of more than 12 KiB."""
+    base = dict(Xdim=16, Ydim=16, Zdim=32, NumProj=4, DeltaAng=90.0)
+    for over in (dict(TAxPixels=2400, TAxPixDim=0.05), dict(AxPixels=300, TAxPixels=300, AxPixDim=0.2, TAxPixDim=0.2)):
+        P = Plan(small_cfg(**{**base, **over}), Options(siddon_bp=SIDDON_BP_GATHER))
+        assert P.quarter_turns and P.mirror_pairs
+        assert back(P) == "bp_gather_quarter_kernel"
+
+
+@pytest.mark.parametrize("name", list(FEW))
+def test_few_views(name):
+    P = Plan(FEW[name], Options(siddon_bp=SIDDON_BP_GATHER))
+    large = FEW[name]["Xdim"] * FEW[name]["Ydim"] >= 16384
+    assert [back(P, n) for n in (1, 2)] == ["bp_gather_few_kernel"] * 2
+    assert [back(P, n) for n in (3, 4)] == ["bp_gather_few_kernel" if large else "bp_gather_pairs_kernel"] * 2
+    assert back(P, 5) == "bp_gather_pairs_kernel"
+    P.bp_view(torch.ones((P.nv, P.nu), device="cuda"), 41.5)
+    assert P.last_kernel(PROJECTOR_BACK) == "bp_gather_few_kernel"
+
+
+def test_other_gathers():
+    # columns a fifth of a voxel: more than four of them meet a voxel column
+    fine = Plan(small_cfg(AxPixels=300, AxPixDim=0.25), Options(siddon_bp=SIDDON_BP_GATHER))
+    assert back(fine, 1) == "bp_gather_pairs_kernel"
+    assert back(Plan(small_cfg(Dz=0.4), Options(siddon_bp=SIDDON_BP_GATHER)), 1) == "bp_gather_kernel"
+    # (pairs of rows come from the column forward projector)
+    assert back(Plan(small_cfg(ZVoxSize=0.05), Options(siddon_bp=SIDDON_BP_GATHER)), 1) == "bp_gather_mirror_kernel"
+
+
+@pytest.mark.parametrize("name", list(RAY))
+def test_ray_design(name):
+    P = Plan(RAY[name], Options(siddon_bp=SIDDON_BP_RAY))
+    assert back(P) == back(P, 1) == iteration(P)[1] == "bp_column_kernel"
+
+
+def test_ray_walk():
+    P = Plan(small_cfg(ZVoxSize=0.05), Options(siddon_bp=SIDDON_BP_RAY))
+    assert back(P) == "bp_ray_kernel" and forward(P) == "fp_kernel"
+    assert iteration(P) == ("fp_kernel", "bp_ray_kernel")
+
+
+@pytest.mark.parametrize("over", [{}, {"Dz": 0.3}])
+def test_forward(over):
+    P = Plan({**BIG, **over})
+    assert forward(P, 5) == "fp_column_wide_kernel" and forward(P) == "fp_column_kernel"
+    assert forward(Plan({**BIG, **over}, Options(sum=SUM_PLAIN)), 5) == "fp_column_kernel"
+    assert forward(Plan({**BIG, **over}, Options(fp_block=32)), 5) == "fp_column_block_kernel"
+
+
+@pytest.mark.parametrize("name", list(VOXEL))
+def test_voxel_update(name):
+    P = Plan(VOXEL[name], Options(bp=BP_VOXEL))
+    staged = name not in ("shorter_image", "dense_rows")
+    assert iteration(P)[1] == ("voxel::bp_staged_kernel" if staged else "voxel::bp_gather_kernel")
+
+
+def test_compat():
+    P = Plan(small_cfg(), Options(arith=ARITH_COMPAT))
+    assert forward(P) == forward(P, 1) == "compat::fp_kernel"
+    assert back(P) == back(P, 1) == "compat::bp_scatter_kernel"
+    assert iteration(P) == ("compat::fp_kernel", "compat::bp_scatter_kernel")
