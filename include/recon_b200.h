@@ -385,9 +385,9 @@ recon_status_t recon_count_intersections(recon_plan_t plan, unsigned long long* 
  * pairs that the forward projector (projector = RECON_PROJECTOR_FORWARD) or
  * the Siddon back projector (RECON_PROJECTOR_BACK) gives a positive length.
  * Equal to recon_count_intersections when no projector drops or adds a pair;
- * where a projector is the ray walk itself (the ray-driven back projector, or
- * the forward walk where the detector-column forward projector does not
- * apply) it is that count.  EXACT arithmetic, synchronous.  A parity check
+ * where a projector is the ray walk itself (the geometries that the
+ * detector-column forward projector does not serve: its forward projector, and
+ * the ray design, ray by ray) it is that count.  EXACT arithmetic, synchronous.  A parity check
  * with no counterpart in the reference. */
 #define RECON_PROJECTOR_FORWARD 0
 #define RECON_PROJECTOR_BACK 1

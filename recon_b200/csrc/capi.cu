@@ -686,8 +686,8 @@ recon_status_t recon_count_projector_pairs(recon_plan_t P, int projector, unsign
     if (projector != RECON_PROJECTOR_FORWARD && projector != RECON_PROJECTOR_BACK)
         return fail(RECON_ERR_INVALID_ARGUMENT, "projector must be RECON_PROJECTOR_FORWARD or RECON_PROJECTOR_BACK");
     RB_CHECK(use_device(*P));
-    // (the ray design along detector columns walks as the column forward projector does)
-    if (P->fp_column && (projector == RECON_PROJECTOR_FORWARD || P->bp_columns)) return exact_fp_column_count(*P, count);
+    if (projector == RECON_PROJECTOR_FORWARD && P->fp_column) return exact_fp_column_count(*P, count);
+    if (projector == RECON_PROJECTOR_BACK && P->bp_columns) return exact_bp_column_count(*P, count);
     if (projector == RECON_PROJECTOR_BACK && P->bp_gather) return exact_bp_gather_count(*P, count);
     return exact_count(*P, count);  // the ray walk, which these projectors run
 }

@@ -703,16 +703,28 @@ constexpr auto fp_column_kernel_of()
 
 // One warp's rows over pieces jb..je; arguments as walk_rows.  With MIRROR the lane's lower
 // row and its mirror (value cvm, at offset Z + 1 - kaddr) share the lengths.
-template <bool FAST, int STEP, bool MIRROR>
-__device__ __forceinline__ void scatter_rows(unsigned long long* acc, const float2* spc, int jb, int je, float cur,
-                                             int kaddr, float kf, float tzn, float S, float O, int step, int kexit, int Z,
-                                             float cv, float cvm)
+// COUNT: nothing is added; the result is the number of pieces of positive length that the
+// lane's rows have inside the volume.
+template <bool FAST, int STEP, bool MIRROR, bool COUNT>
+__device__ __forceinline__ unsigned scatter_rows(unsigned long long* acc, const float2* spc, int jb, int je, float cur,
+                                                 int kaddr, float kf, float tzn, float S, float O, int step, int kexit,
+                                                 int Z, float cv, float cvm)
 {
     const int st = STEP != 0 ? STEP : step;
     const float fst = (float)st;
+    unsigned pieces = 0;
     auto add = [](unsigned long long* p, float x) {
         const long long q = __float2ll_rn(x);
         if (q != 0) atomicAdd(p, (unsigned long long)q);
+    };
+    // the stretch L of a piece in layer k - 1 (both rows: a mirror row's layer is inside when its row's is)
+    auto take = [&](unsigned long long* col, int k, float L) {
+        if constexpr (COUNT) {
+            if (L > 0.0f && (unsigned)(k - 1) < (unsigned)Z) pieces += MIRROR ? 2u : 1u;
+        } else {
+            add(col + k, L * cv);
+            if (MIRROR) add(col + (Z + 1 - k), L * cvm);
+        }
     };
 #pragma unroll 4
     for (int j = jb; j <= je; ++j) {
@@ -721,26 +733,26 @@ __device__ __forceinline__ void scatter_rows(unsigned long long* acc, const floa
         unsigned long long* const col = acc + __float_as_int(pc.y);
         const bool cross = tzn < B;
         const float m = fminf(tzn, B), L0 = m - cur;
-        add(col + kaddr, L0 * cv);
-        if (MIRROR) add(col + (Z + 1 - kaddr), L0 * cvm);
+        take(col, kaddr, L0);
         if (cross) {
             kaddr += st;
             const float L1 = B - m;
-            add(col + kaddr, L1 * cv);
-            if (MIRROR) add(col + (Z + 1 - kaddr), L1 * cvm);
+            take(col, kaddr, L1);
             kf += fst;
             tzn = fmaf(kf, S, O);
             if (!FAST && kaddr == kexit) tzn = __int_as_float(0x7f800000);
         }
         cur = B;
     }
+    return pieces;
 }
 
 // Detector columns as the forward kernel takes them (tiles, or the full grid from row v0),
 // each path in nseg stretches, one per block (blockIdx.y of a tile, blockIdx.z % nseg).
 // vals: values times w in detector columns [view - view0][u][v], with view_stride 0 one table
 // for every view, or with wq a sinogram's values [view - view0][v][u], still to be weighted.
-template <bool MIRROR>
+// COUNT: the (ray, voxel) pairs of positive length, over every row, into acc[0].
+template <bool MIRROR, bool COUNT>
 __global__ void __launch_bounds__(kColRows) bp_column_kernel(ExactGeom G, const float4* __restrict__ txy,
                                                              const int2* __restrict__ kxy, const ZParam* __restrict__ zp,
                                                              const uint2* __restrict__ tiles, unsigned view0, int v0,
@@ -752,7 +764,7 @@ __global__ void __launch_bounds__(kColRows) bp_column_kernel(ExactGeom G, const 
 {
     extern __shared__ float2 spc[];
     __shared__ float scale_s;
-    if (threadIdx.x == 0) scale_s = fix_scale_of(__ldg(maxabs), max_len, count_bits).scale;
+    if (threadIdx.x == 0) scale_s = COUNT ? 1.0f : fix_scale_of(__ldg(maxabs), max_len, count_bits).scale;
     unsigned view;
     int u, vstart;
     if (tiles) {
@@ -772,6 +784,7 @@ __global__ void __launch_bounds__(kColRows) bp_column_kernel(ExactGeom G, const 
     // the value(s) of the lane's row(s): every load before any is used
     const size_t base = (size_t)(view - view0) * view_stride, pc = (size_t)u * G.Nv;
     auto value = [&](int row) {
+        if (COUNT) return 1.0f;
         if (wq) return __ldg(valsf + base + (size_t)row * G.Nu + u) * __ldg(wq + pc + row);
         return valsf ? __ldg(valsf + base + pc + row) : load_val<__nv_bfloat16>(valsb + base + pc + row);
     };
@@ -793,13 +806,18 @@ __global__ void __launch_bounds__(kColRows) bp_column_kernel(ExactGeom G, const 
                              : row_walk(G, zp, spc, n, t_in, t_out, v, valid && cv != 0.0f, jlo, jhi);
     if (W.jb > W.je) return;  // no row of the warp crosses the volume with a value
     const float a = W.hit ? cv : 0.0f, am = W.hit ? cvm : 0.0f;
+    unsigned pieces;
     if (MIRROR) {
-        if (W.fast) scatter_rows<true, -1, true>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, -1, 0, G.Z, a, am);
-        else scatter_rows<false, -1, true>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, -1, 0, G.Z, a, am);
+        if (W.fast) pieces = scatter_rows<true, -1, true, COUNT>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, -1, 0, G.Z, a, am);
+        else pieces = scatter_rows<false, -1, true, COUNT>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, -1, 0, G.Z, a, am);
     } else if (W.fast) {
-        scatter_rows<true, 0, false>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, W.dk, W.kexit, G.Z, a, am);
+        pieces = scatter_rows<true, 0, false, COUNT>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, W.dk, W.kexit, G.Z, a, am);
     } else {
-        scatter_rows<false, 0, false>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, W.dk, W.kexit, G.Z, a, am);
+        pieces = scatter_rows<false, 0, false, COUNT>(acc, spc, W.jb, W.je, W.t_start, W.kaddr, W.kf, W.tzn, W.S, W.O, W.dk, W.kexit, G.Z, a, am);
+    }
+    if (COUNT) {
+        pieces = __reduce_add_sync(0xffffffffu, W.hit ? pieces : 0u);
+        if ((threadIdx.x & 31u) == 0u && pieces) atomicAdd(acc, (unsigned long long)pieces);
     }
 }
 
@@ -1314,6 +1332,45 @@ static recon_status_t launch_column(Plan& P, const float* vol, unsigned first, u
 
 constexpr int kStretch = 32;  // voxels of x + y a stretch, at least
 
+// bp_column_kernel over views [first, first + count) of table slots: what it adds to and
+// scales by as its parameters, or with COUNT the pairs into acc[0].
+template <bool COUNT>
+static recon_status_t launch_bp_column(Plan& P, unsigned first, unsigned count, const float* vf, const __nv_bfloat16* vb,
+                                       size_t view_stride, const float* wq, float max_len, int cbits,
+                                       unsigned long long* acc, cudaStream_t s)
+{
+    const ExactGeom& E = P.eg;
+    const size_t smem = (size_t)(E.X + E.Y + 2) * sizeof(float2);
+    auto kernel = P.z_mirror ? exact::bp_column_kernel<true, COUNT> : exact::bp_column_kernel<false, COUNT>;
+    note_kernel(RECON_PROJECTOR_BACK, "bp_column_kernel");
+    if (smem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, kPathSmem));
+    auto launch = [&](dim3 grid, int rows, const uint2* tiles, int v0) -> recon_status_t {
+        // a launch of few warps takes the paths in stretches (the sums do not care)
+        const double warps = (double)grid.x * grid.y * grid.z * (rows / 32);
+        const double most = std::max(1, (E.X + E.Y) / kStretch);  // pieces enough to be worth finding the path
+        const int nseg = (int)std::min({8.0, most, std::max(1.0, 32.0 * P.sm_count / warps)});
+        if (tiles) grid.y *= nseg;
+        else grid.z *= nseg;
+        kernel<<<grid, rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, tiles, first, v0, nseg, vf, vb, view_stride, wq, P.d_bpmax,
+                                        max_len, cbits, acc);
+        RB_CUDA(cudaGetLastError());
+        return RECON_OK;
+    };
+    const int rows = P.z_mirror ? E.Nv / 2 : E.Nv;
+    if (count > 24 && bp_acc_words(P) * sizeof(unsigned long long) > (size_t(115) << 20)) {
+        // an accumulator that the 126 MB L2 does not hold: 32 rows of every view at a time,
+        // whose rays meet a slab of it (256^3, 120 views: 3.45 against 5.4 ms by views; at
+        // 240^3, 113 MB, by views 2.8 against 2.95 ms; ten views are faster by views)
+        for (int v0 = 0; v0 < rows; v0 += 32) RB_CHECK(launch(dim3(E.Nu, 1, count), 32, nullptr, v0));
+    } else if (first + count <= P.nviews && P.col_tiles.prefix.size() == P.nviews + 1) {
+        const unsigned t0 = P.col_tiles.prefix[first], nt = P.col_tiles.prefix[first + count] - t0;
+        if (nt) RB_CHECK(launch(dim3(nt, 1, 1), P.col_rows, P.col_tiles.d + t0, 0));
+    } else {
+        RB_CHECK(launch(dim3(E.Nu, (rows + P.col_rows - 1) / P.col_rows, count), P.col_rows, nullptr, 0));
+    }
+    return RECON_OK;
+}
+
 // The ray design's back projection along detector columns: views [first, first + count) of
 // table slots, vals as bp_column_kernel takes them, vmax[0 .. nmax) the views' largest
 // magnitudes (found here for a sinogram that is still to be weighted, wq); vol = Ht, or with
@@ -1332,38 +1389,11 @@ recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, const flo
                                                   sino_max ? 0u : nmax, P.d_bpmax);
     RB_CUDA(cudaGetLastError());
     if (sino_max) RB_CHECK(launch_maxabs(P, (const float*)vals, count, P.d_bpmax, s));
-    const size_t smem = (size_t)(E.X + E.Y + 2) * sizeof(float2);
-    auto kernel = P.z_mirror ? exact::bp_column_kernel<true> : exact::bp_column_kernel<false>;
-    note_kernel(RECON_PROJECTOR_BACK, "bp_column_kernel");
-    if (smem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, kPathSmem));
     const float* vf = nullptr;
     const __nv_bfloat16* vb = nullptr;
     if constexpr (std::is_same<ST, float>::value) vf = vals;
     else vb = vals;
-    auto launch = [&](dim3 grid, int rows, const uint2* tiles, int v0) -> recon_status_t {
-        // a launch of few warps takes the paths in stretches (the sums do not care)
-        const double warps = (double)grid.x * grid.y * grid.z * (rows / 32);
-        const double most = std::max(1, (E.X + E.Y) / kStretch);  // pieces enough to be worth finding the path
-        const int nseg = (int)std::min({8.0, most, std::max(1.0, 32.0 * P.sm_count / warps)});
-        if (tiles) grid.y *= nseg;
-        else grid.z *= nseg;
-        kernel<<<grid, rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, tiles, first, v0, nseg, vf, vb, view_stride, wq, P.d_bpmax,
-                                        max_len, cbits, P.d_bpacc);
-        RB_CUDA(cudaGetLastError());
-        return RECON_OK;
-    };
-    const int rows = P.z_mirror ? E.Nv / 2 : E.Nv;
-    if (count > 24 && bp_acc_words(P) * sizeof(unsigned long long) > (size_t(115) << 20)) {
-        // an accumulator that the 126 MB L2 does not hold: 32 rows of every view at a time,
-        // whose rays meet a slab of it (256^3, 120 views: 3.45 against 5.4 ms by views; at
-        // 240^3, 113 MB, by views 2.8 against 2.95 ms; ten views are faster by views)
-        for (int v0 = 0; v0 < rows; v0 += 32) RB_CHECK(launch(dim3(E.Nu, 1, count), 32, nullptr, v0));
-    } else if (first + count <= P.nviews && P.col_tiles.prefix.size() == P.nviews + 1) {
-        const unsigned t0 = P.col_tiles.prefix[first], nt = P.col_tiles.prefix[first + count] - t0;
-        if (nt) RB_CHECK(launch(dim3(nt, 1, 1), P.col_rows, P.col_tiles.d + t0, 0));
-    } else {
-        RB_CHECK(launch(dim3(E.Nu, (rows + P.col_rows - 1) / P.col_rows, count), P.col_rows, nullptr, 0));
-    }
+    RB_CHECK(launch_bp_column<false>(P, first, count, vf, vb, view_stride, wq, max_len, cbits, P.d_bpacc, s));
     const dim3 fgrid((unsigned)((E.X + 31) / 32) * (unsigned)((E.Z + 31) / 32), std::min(E.Y, 65535));
     if (sens)
         exact::bp_column_finish_kernel<2><<<fgrid, dim3(32, 8), 0, s>>>(E, P.d_bpmax, max_len, cbits, P.d_bpacc, vol, sens);
@@ -1377,21 +1407,37 @@ template recon_status_t bp_columns<float>(Plan&, const float*, size_t, const flo
 template recon_status_t bp_columns<__nv_bfloat16>(Plan&, const __nv_bfloat16*, size_t, const float*, unsigned,
                                                   unsigned, const unsigned*, unsigned, float*, const float*, cudaStream_t);
 
-// (ray, voxel) pairs of positive length over all plan views, as the column
-// kernel assigns them (synchronous; no volume is read).
-recon_status_t exact_fp_column_count(Plan& P, unsigned long long* total)
+// The pairs that one of the column walks counts into a device word (synchronous).
+template <class Count>
+static recon_status_t count_column_pairs(unsigned long long* total, Count count)
 {
     unsigned long long* d = nullptr;
     RB_CUDA(cudaMalloc(&d, sizeof(unsigned long long)));
     cudaError_t e = cudaMemset(d, 0, sizeof(unsigned long long));
-    recon_status_t st = RECON_OK;
-    if (e == cudaSuccess)
-        st = launch_column<3, kLayoutRows, float, unsigned long long>(P, nullptr, 0u, P.nviews, nullptr, d, 0);
+    recon_status_t st = e == cudaSuccess ? count(d) : RECON_OK;
     if (e == cudaSuccess && st == RECON_OK) e = cudaMemcpy(total, d, sizeof(unsigned long long), cudaMemcpyDeviceToHost);
     cudaFree(d);
     if (st != RECON_OK) return st;
     if (e != cudaSuccess) return cuda_fail(e, "column pair count");
     return RECON_OK;
+}
+
+// (ray, voxel) pairs of positive length over all plan views, as the column
+// kernel assigns them (no volume is read).
+recon_status_t exact_fp_column_count(Plan& P, unsigned long long* total)
+{
+    return count_column_pairs(total, [&](unsigned long long* d) {
+        return launch_column<3, kLayoutRows, float, unsigned long long>(P, nullptr, 0u, P.nviews, nullptr, d, 0);
+    });
+}
+
+// The same of the ray design along detector columns, launched as it back projects all of
+// the plan's views.
+recon_status_t exact_bp_column_count(Plan& P, unsigned long long* total)
+{
+    return count_column_pairs(total, [&](unsigned long long* d) {
+        return P.nviews ? launch_bp_column<true>(P, 0u, P.nviews, nullptr, nullptr, 0, nullptr, 0.0f, 0, d, 0) : RECON_OK;
+    });
 }
 
 recon_status_t exact_fp_column(Plan& P, const float* vol, unsigned first, unsigned count, float* out, cudaStream_t s)

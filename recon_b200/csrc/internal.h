@@ -240,6 +240,7 @@ recon_status_t exact_fp_ratio(Plan& P, const float* vol, const void* g, void* ra
 recon_status_t exact_count(Plan& P, unsigned long long* out);
 recon_status_t exact_bp_gather_count(Plan& P, unsigned long long* total);
 recon_status_t exact_fp_column_count(Plan& P, unsigned long long* total);
+recon_status_t exact_bp_column_count(Plan& P, unsigned long long* total);
 // BP gather over views [first, first+count) of `sino` (weighted by w) into vol (overwrite);
 // sens_mode: back project ones; update: f = f*Ht/sens in the epilogue.
 recon_status_t exact_bp(Plan& P, const void* sino, bool sino_is_rw, bool bf16, unsigned first,
