@@ -320,18 +320,9 @@ recon_status_t recon_plan_create(const recon_geometry_t* geom, const recon_optio
                 exact_use_gather(*P, true);
                 if (P->col_pairs) RB_CHECK(build_wq_pairs(*P));
             }
-            if (!gather) exact_use_gather(*P, false);
-            if (P->bp_columns) {
-                RB_CHECK(build_view_maxima(*P));
-                RB_CHECK(P->alloc(&P->d_bpacc, bp_acc_words(*P) + 1, "back projection accumulator"));  // cleared in pairs
-                RB_CHECK(P->alloc(&P->d_bpmax, 1, "back projection max"));
-            } else if (!gather) {  // the ray-driven back projector's slab accumulators
-                const size_t slab = (size_t)P->eg.X * P->eg.Y * bp_slab_depth(*P);
-                RB_CHECK(P->alloc(&P->d_bpacc, slab, "back projection accumulator"));
-                RB_CHECK(P->alloc(&P->d_bpacc_t, slab, "back projection accumulator (transposed)"));
-                RB_CHECK(P->alloc(&P->d_bpmax, 1, "back projection max"));
-                RB_CUDA(cudaMemset(P->d_bpacc, 0, slab * sizeof(unsigned long long)));
-                RB_CUDA(cudaMemset(P->d_bpacc_t, 0, slab * sizeof(unsigned long long)));
+            if (!gather) {
+                exact_use_gather(*P, false);
+                RB_CHECK(exact_alloc_ray(*P));
             }
             RB_CHECK(build_exact_culling(*P));
             if (tuned) RB_CHECK(exact_tune_bp(*P));

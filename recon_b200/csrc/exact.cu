@@ -1869,7 +1869,7 @@ void plan_release(Plan& P, void* p, size_t bytes)
 
 // Times the plan's sensitivity back projection (all views, both designs set up
 // by the plan) with each design, CUDA events around the second of two runs on
-// the legacy stream, and keeps the faster; the ray design's slab accumulators
+// the legacy stream, and keeps the faster; the ray design's accumulators
 // are released when the gather wins.  Synchronous (plan creation).
 recon_status_t exact_tune_bp(Plan& P)
 {
@@ -2188,7 +2188,7 @@ recon_status_t build_wq_pairs(Plan& P)
 }
 
 // The ray design's view maxima (bp_columns), the weights' among them.
-recon_status_t build_view_maxima(Plan& P)
+static recon_status_t build_view_maxima(Plan& P)
 {
     const size_t n = (size_t)P.nviews + 1;
     RB_CHECK(P.alloc(&P.d_vmax, n, "view maxima"));
@@ -2222,8 +2222,43 @@ size_t bp_acc_words(const Plan& P) { return (size_t)P.eg.X * P.eg.Y * (P.eg.Z + 
 void exact_use_gather(Plan& P, bool gather)
 {
     P.bp_gather = gather;
-    P.bp_columns = !gather && P.fp_column && bp_acc_words(P) <= (size_t(1) << 29);
+    P.bp_columns = !gather && P.fp_column && !P.bp_no_room && bp_acc_words(P) <= (size_t(1) << 29);
     P.col_pairs = gather && exact_pairs_suit(P);
+}
+
+// The ray design's accumulators: the whole volume's (8 bytes a voxel) along detector
+// columns, else two of a slab of at most 64 MiB together.  A device without room for the
+// first and the buffers that an MLEM iteration will add (looked at where the first takes
+// more than the slabs would) gets the second, which give the same bits more slowly.
+recon_status_t exact_alloc_ray(Plan& P)
+{
+    if (P.bp_columns) {
+        const size_t words = bp_acc_words(P) + 1;  // cleared in pairs
+        bool room = true;
+        if (words * sizeof(unsigned long long) > size_t(64) << 20) {
+            size_t free_bytes = 0, total = 0;
+            RB_CUDA(cudaMemGetInfo(&free_bytes, &total));
+            const size_t iteration = P.nvox * sizeof(float) +
+                                     (size_t)P.nviews * P.npix * (P.opt.sino == RECON_SINO_BF16 ? 2 : 4);
+            room = words * sizeof(unsigned long long) + iteration <= free_bytes;
+        }
+        const recon_status_t st =
+            room ? P.alloc(&P.d_bpacc, words, "back projection accumulator") : RECON_ERR_OUT_OF_MEMORY;
+        if (st == RECON_OK) {
+            RB_CHECK(build_view_maxima(P));
+            return P.alloc(&P.d_bpmax, 1, "back projection max");
+        }
+        if (st != RECON_ERR_OUT_OF_MEMORY) return st;
+        P.bp_no_room = true;
+        exact_use_gather(P, false);
+    }
+    const size_t slab = (size_t)P.eg.X * P.eg.Y * bp_slab_depth(P);
+    RB_CHECK(P.alloc(&P.d_bpacc, slab, "back projection accumulator"));
+    RB_CHECK(P.alloc(&P.d_bpacc_t, slab, "back projection accumulator (transposed)"));
+    RB_CHECK(P.alloc(&P.d_bpmax, 1, "back projection max"));
+    RB_CUDA(cudaMemset(P.d_bpacc, 0, slab * sizeof(unsigned long long)));
+    RB_CUDA(cudaMemset(P.d_bpacc_t, 0, slab * sizeof(unsigned long long)));
+    return RECON_OK;
 }
 
 // Views of a sinogram [view][v][u] times w into the gather's input d_colsino.

@@ -136,6 +136,7 @@ struct Plan {
     unsigned colsino_views = 0;   // views d_colsino holds
     bool bp_gather = false;    // Siddon back projection by the column gather (else the ray design)
     bool bp_columns = false;   // the ray design along detector columns (else ray by ray in slabs)
+    bool bp_no_room = false;   // the device had no room for bp_columns' accumulator
     unsigned* d_vmax = nullptr;  // bp_columns: max |value| (float bits) of the ratio's views [nviews], then of
                                  // the weights
     bool z_mirror = false;     // z table mirror-symmetric about z = 0: both projectors pair mirrored rows/voxels
@@ -294,7 +295,7 @@ int exact_column_rows_default(const Plan& P, const std::vector<int4>& rect);
 std::string geometry_key(const Plan& P);
 void plan_release(Plan& P, void* p, size_t bytes);
 recon_status_t build_wq_pairs(Plan& P);
-recon_status_t build_view_maxima(Plan& P);
+recon_status_t exact_alloc_ray(Plan& P);
 void exact_use_gather(Plan& P, bool gather);
 size_t bp_acc_words(const Plan& P);
 recon_status_t launch_maxabs(Plan& P, const float* sino, unsigned count, unsigned* out, cudaStream_t s);
