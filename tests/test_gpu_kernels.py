@@ -67,6 +67,21 @@ def test_few_views(name):
     assert P.last_kernel(PROJECTOR_BACK) == "bp_gather_few_kernel"
 
 
+def test_large_detectors():
+    """Up to 4096 rows and 8192 columns the few-view gather's bounds hold; it drops no ray there."""
+    for rows, columns in ((4096, 64), (4098, 64), (48, 8192), (48, 8193)):
+        cfg = small_cfg(TAxPixels=rows, TAxPixDim=72.0 / rows, AxPixels=columns, AxPixDim=96.0 / min(columns, 96))
+        P = Plan(cfg, Options(siddon_bp=SIDDON_BP_GATHER))
+        y = torch.rand((1, P.nv, P.nu), device="cuda", generator=torch.Generator("cuda").manual_seed(341))
+        out = P.bp_views(y, 3, 1)
+        small = rows <= 4096 and columns <= 8192
+        assert P.last_kernel(PROJECTOR_BACK) == ("bp_gather_few_kernel" if small else "bp_gather_pairs_kernel")
+        exact = Plan(cfg, Options(siddon_bp=SIDDON_BP_RAY)).bp_views(y, 3, 1)
+        # FP32 sums of at most a few hundred products a voxel against exact ones
+        assert ((out - exact).norm() / exact.norm()).item() < 2e-6
+        assert torch.equal(out != 0, exact != 0)
+
+
 def test_other_gathers():
     # columns a fifth of a voxel: more than four of them meet a voxel column
     fine = Plan(small_cfg(AxPixels=300, AxPixDim=0.25), Options(siddon_bp=SIDDON_BP_GATHER))
