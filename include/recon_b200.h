@@ -190,6 +190,15 @@ recon_status_t recon_plan_create(const recon_geometry_t* geom, const recon_optio
 /* Replaces siddon_commons::a3_deallocate and the class destructors
  * (hf_siddon_class.hpp:109-132, 232-244, 354-368; hf_siddon_recon.hpp:594-606). */
 void recon_plan_destroy(recon_plan_t plan);
+/* Waits for the stream, then returns RECON_ERR_CUDA where a kernel of the plan has given up
+ * a wait for an asynchronous copy (about two seconds without an answer; its results are NaN),
+ * or reports an error of the stream's work.  Any later call on the plan reports a wait that
+ * was given up too; each is reported once, and the plan stays usable.  Not to be called while
+ * the stream is capturing. */
+recon_status_t recon_plan_check(recon_plan_t plan, void* stream);
+/* Makes such a wait run out after about ten milliseconds, on a barrier that nothing completes,
+ * for tests of the report.  RECON_ERR_UNSUPPORTED for plans whose kernels have no such waits. */
+recon_status_t recon_selftest_wait(recon_plan_t plan, void* stream);
 /* Device bytes held by the plan. */
 size_t recon_plan_device_bytes(recon_plan_t plan);
 /* The Siddon back projector an EXACT plan uses (RECON_SIDDON_BP_GATHER or

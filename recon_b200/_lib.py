@@ -102,6 +102,8 @@ def lib() -> C.CDLL:
         "recon_plan_create": (st, [C.POINTER(Geometry), C.POINTER(Options), C.POINTER(P)]),
         "recon_plan_destroy": (None, [P]),
         "recon_plan_device_bytes": (C.c_size_t, [P]),
+        "recon_plan_check": (st, [P, P]),
+        "recon_selftest_wait": (st, [P, P]),
         "recon_plan_siddon_bp": (st, [P, ip]),
         "recon_plan_forward_projector": (st, [P, C.POINTER(C.c_int)]),
         "recon_plan_mirror_pairs": (st, [P, C.POINTER(C.c_int)]),
@@ -164,7 +166,7 @@ def exported_symbols() -> list[str]:
         "recon_add", "recon_compat_setup_view", "recon_compat_trace", "recon_view_step_count", "recon_mlem_from_cfg",
         "recon_forward_projection_from_cfg", "recon_backward_projection_from_cfg", "recon_batch_create",
         "recon_batch_destroy", "recon_batch_mlem", "recon_compat_bp_view_noalloc", "recon_osem",
-        "recon_upload_sinogram", "recon_last_kernel",
+        "recon_upload_sinogram", "recon_last_kernel", "recon_plan_check", "recon_selftest_wait",
     ]
 
 

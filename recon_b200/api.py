@@ -191,6 +191,11 @@ class Plan:
 
         return torch.empty(shape, dtype=torch.float32, device=f"cuda:{self.options.device}")
 
+    def check(self) -> None:
+        """Waits for the current stream and raises where the plan's work on it failed
+        (recon_plan_check)."""
+        check(lib().recon_plan_check(self._h, _stream()))
+
     # --- projectors ---
     def fp_view(self, vol, angle: float, out=None):
         out = self._empty((self.nv, self.nu)) if out is None else out

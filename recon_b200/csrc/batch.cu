@@ -243,6 +243,7 @@ recon_status_t recon_batch_mlem(recon_batch_t b, const float* const* d_g, float*
     const size_t n = b->plans.size();
     for (size_t p = 0; p < n; ++p)
         if (!d_g[p] || !d_f[p]) return fail(RECON_ERR_INVALID_ARGUMENT, "NULL problem buffer");
+    for (auto plan : b->plans) RB_CHECK(take_give_up(*plan));
     RB_CUDA(cudaSetDevice(b->device));
     cudaStream_t s = as_stream(stream), origin = b->streams[0];
     // the work runs on the graph's stream, ordered after the caller's stream

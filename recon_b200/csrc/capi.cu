@@ -37,6 +37,7 @@ Plan::~Plan()
     release_plan_textures(this);
     if (vol_z_free) cudaEventDestroy(vol_z_free);
     for (void* p : allocations) cudaFree(p);
+    if (h_give_up) cudaFreeHost(h_give_up);
     if (cur >= 0 && cur != device) cudaSetDevice(cur);
 }
 
@@ -171,12 +172,21 @@ static void fill_geoms(Plan& P)
     E.vd0 = (float)(-((double)C.Nv - 1.0) / 2.0 * dv);
 }
 
-static recon_status_t use_device(const Plan& P)
+// An earlier call's kernel gave up a wait: reported once.
+recon_status_t take_give_up(Plan& P)
+{
+    if (!P.h_give_up || !*(volatile unsigned*)P.h_give_up) return RECON_OK;
+    *(volatile unsigned*)P.h_give_up = 0u;
+    return fail(RECON_ERR_CUDA, "a wait for an asynchronous copy ran out in an earlier call of this plan: the results "
+                                "since are not valid");
+}
+
+static recon_status_t use_device(Plan& P)
 {
     int cur = -1;
     RB_CUDA(cudaGetDevice(&cur));
     if (cur != P.device) RB_CUDA(cudaSetDevice(P.device));
-    return RECON_OK;
+    return take_give_up(P);
 }
 
 // Index of a plan view whose angle equals `angle` exactly, else -1.
@@ -318,6 +328,11 @@ recon_status_t recon_plan_create(const recon_geometry_t* geom, const recon_optio
             const bool gather = P->bp_gather && !tuned;
             if (gather || tuned) {
                 exact_use_gather(*P, true);
+                if (P->quarter) {  // the staged gather waits for its copies
+                    RB_CUDA(cudaHostAlloc((void**)&P->h_give_up, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable));
+                    *P->h_give_up = 0u;
+                    RB_CUDA(cudaHostGetDevicePointer((void**)&P->d_give_up, P->h_give_up, 0));
+                }
                 if (P->col_pairs) RB_CHECK(build_wq_pairs(*P));
             }
             if (!gather) {
@@ -351,6 +366,22 @@ recon_status_t recon_plan_create(const recon_geometry_t* geom, const recon_optio
 void recon_plan_destroy(recon_plan_t plan) { delete plan; }
 
 size_t recon_plan_device_bytes(recon_plan_t plan) { return plan ? plan->device_bytes : 0; }
+
+recon_status_t recon_plan_check(recon_plan_t P, void* stream)
+{
+    if (!P) return fail(RECON_ERR_INVALID_ARGUMENT, "NULL plan");
+    RB_CHECK(use_device(*P));
+    RB_CUDA(cudaStreamSynchronize(as_stream(stream)));
+    return take_give_up(*P);
+}
+
+recon_status_t recon_selftest_wait(recon_plan_t P, void* stream)
+{
+    if (!P) return fail(RECON_ERR_INVALID_ARGUMENT, "NULL plan");
+    RB_CHECK(use_device(*P));
+    if (!P->d_give_up) return fail(RECON_ERR_UNSUPPORTED, "the plan's kernels wait for no asynchronous copies");
+    return launch_wait_selftest(*P, as_stream(stream));
+}
 
 recon_status_t recon_plan_forward_projector(recon_plan_t plan, int* design)
 {

@@ -430,6 +430,7 @@ recon_status_t recon_mlem_from_cfg(const char* folder, const char* cfg, const re
     for (unsigned it = L.start_iteration; it < g.scan.N_iteration; ++it) {
         RB_TRY(recon_mlem_iteration(plan.p, d_g.p, d_f.p, nullptr));
         RB_TRY(to_host(f.data(), d_f.p, nvox));
+        RB_TRY(recon_plan_check(plan.p, nullptr));
         RB_TRY(write_floats(numbered(L.paths.ReconFileFolder, L.paths.ReconFileNameRoot, it, L.paths.ReconFileSuffix),
                             f.data(), nvox));
     }

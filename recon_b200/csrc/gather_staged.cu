@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
     ExactGeom G, GatherConst C, StagedShape S, const float4* __restrict__ txy, const int2* __restrict__ kxy,
     const float2* __restrict__ cs, const ZParam* __restrict__ zp, unsigned nview, unsigned m0, unsigned mc,
     const __grid_constant__ CUtensorMap vals, unsigned view_rows, float* __restrict__ vol,
-    const float* __restrict__ sens, unsigned long long* __restrict__ npairs)
+    const float* __restrict__ sens, unsigned long long* __restrict__ npairs, unsigned* give_up)
 {
     constexpr unsigned kPair = 2 * sizeof(ST);  // bytes of a pair
     constexpr int NE = 8 * PS * 32;  // epilogue entries per warp
@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
                     }
                 }
                 if (!ok) {  // a warp does not answer: let the copies in flight land, then stop
+                    if (lane == 0) report_give_up(give_up);
                     for (unsigned b = 1; b <= min(n, (unsigned)S.stages); ++b) {
                         const unsigned use = base + n - b;
                         mbar_wait(smem_addr(&full[use % (unsigned)S.stages]), (use / (unsigned)S.stages) & 1u);
@@ -250,6 +251,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
                 __syncwarp();  // the next batch rewrites the items
             }
             if (!ok) {  // a stage never came: the sums are not the answer
+                if (lane == 0) report_give_up(give_up);
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -312,9 +314,25 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
     }
 }
 
+// A wait on a barrier that nothing arrives at, with a limit of about ten milliseconds.
+__global__ void wait_selftest_kernel(unsigned* give_up)
+{
+    __shared__ unsigned long long bar;
+    mbar_init(smem_addr(&bar), 1u);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (!mbar_wait(smem_addr(&bar), 0u, 20000000ll)) report_give_up(give_up);
+}
+
 }  // namespace exact
 
 // ---- host side -----------------------------------------------------------------------------
+
+recon_status_t launch_wait_selftest(Plan& P, cudaStream_t s)
+{
+    exact::wait_selftest_kernel<<<1, 1, 0, s>>>(P.d_give_up);
+    RB_CUDA(cudaGetLastError());
+    return RECON_OK;
+}
 
 // Detector columns whose rays can meet a rectangle of diagonal d mm anywhere in the
 // volume: its shadow is at most d * |Ry| / depth * sqrt(1 + tan^2) / du pitches wide.
@@ -446,7 +464,7 @@ static recon_status_t launch_staged(Plan& P, const exact::StagedShape& S, size_t
     const int H = E.X / 2;
     const dim3 grid((H + exact::kStagedTX - 1) / exact::kStagedTX, (H + exact::kStagedTY - 1) / exact::kStagedTY);
     kernel<<<grid, exact::kStagedThreads, smem, s>>>(E, gather_const(P, vol, sens), S, P.d_txy, P.d_kxy, P.d_cs, P.d_zp,
-                                                     P.nviews, m0, mc, map, view_rows, vol, sens, npairs);
+                                                     P.nviews, m0, mc, map, view_rows, vol, sens, npairs, P.d_give_up);
     RB_CUDA(cudaGetLastError());
     return RECON_OK;
 }
@@ -474,7 +492,7 @@ recon_status_t staged_quarter_gather(Plan& P, const ST* vals, size_t view_stride
     // view_stride 0: the same table for every view (the weights of the sensitivity)
     const unsigned view_rows = view_stride ? (unsigned)P.eg.Nu : 0u;
     const size_t table_rows = view_stride ? (size_t)P.eg.Nu * P.nviews : (size_t)P.eg.Nu;
-    *served = table_rows < 0x7fffffff && staged_shape(P, slots, sizeof(ST), &S, &region, &smem) &&
+    *served = P.d_give_up && table_rows < 0x7fffffff && staged_shape(P, slots, sizeof(ST), &S, &region, &smem) &&
               column_map(S, vals, pair_entries(P.eg.Nv), 2 * sizeof(ST), table_rows, &map);
     if (!*served) return RECON_OK;
     auto run = [&](auto ps) -> recon_status_t {

@@ -60,15 +60,21 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity)
         : "memory");
     return done != 0u;
 }
-// Waits until the barrier's phase of this parity is complete; gives up after about
-// two seconds (false), which no run that works comes near.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity)
+// Waits until the barrier's phase of this parity is complete; gives up after `limit` clocks
+// (false), by default about two seconds, which no run that works comes near.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, long long limit = 4000000000ll)
 {
     if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try(bar, parity))
-        if (clock64() - t0 > 4000000000ll) return false;
+        if (clock64() - t0 > limit) return false;
     return true;
+}
+// A wait was given up: the plan's word in host memory says so to its next call.
+__device__ __forceinline__ void report_give_up(unsigned* word)
+{
+    *(volatile unsigned*)word = 1u;
+    __threadfence_system();
 }
 // The box at entry x (a multiple of four) of table row y into dst (128-byte aligned).
 __device__ __forceinline__ void tile_load(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar)

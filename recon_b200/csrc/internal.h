@@ -189,6 +189,10 @@ struct Plan {
     unsigned long long* d_fix = nullptr;  // COMPAT: fixed-point accumulator [nvox]
     unsigned* d_maxabs = nullptr; // COMPAT: max |value| bits per view, scratch slot, several views [nviews+2]
     float* d_view_img = nullptr;  // scratch image [npix]
+    // host word, and its device address, that a kernel sets when one of its waits on an
+    // asynchronous copy ran out (plans whose back projector has such waits)
+    unsigned* h_give_up = nullptr;
+    unsigned* d_give_up = nullptr;
     size_t device_bytes = 0;
     std::vector<void*> allocations;
 
@@ -267,6 +271,7 @@ recon_status_t plain_fp_ratio(Plan& P, const float* vol, const float* g, float* 
 recon_status_t exact_fp_plain_ratio(Plan& P, const float* vol, const float* g, float* ratio, cudaStream_t s);
 recon_status_t compat_fp_ratio_all(Plan& P, const float* vol, const float* g, float* ratio, cudaStream_t s);
 void release_plan_textures(Plan* P);
+recon_status_t take_give_up(Plan& P);
 recon_status_t ensure_mlem_buffers(Plan& P);
 recon_status_t compute_sensitivity(Plan& P, float* sens, cudaStream_t s);
 recon_status_t describe_compat_geometry(const recon_geometry_t& g, Plan& P);
@@ -296,6 +301,7 @@ std::string geometry_key(const Plan& P);
 void plan_release(Plan& P, void* p, size_t bytes);
 recon_status_t build_wq_pairs(Plan& P);
 recon_status_t exact_alloc_ray(Plan& P);
+recon_status_t launch_wait_selftest(Plan& P, cudaStream_t s);
 void exact_use_gather(Plan& P, bool gather);
 size_t bp_acc_words(const Plan& P);
 recon_status_t launch_maxabs(Plan& P, const float* sino, unsigned count, unsigned* out, cudaStream_t s);
