@@ -106,16 +106,16 @@ __device__ __forceinline__ float as_stored<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ float as_stored<__nv_bfloat16>(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-// *slot = max(*slot, the calling lanes' largest |value| as float bits): one atomic for the
-// active lanes of a warp, which nothing waits for.
-__device__ __forceinline__ void raise_max(unsigned* slot, float value)
+// *slot = max(*slot, the largest |value| of the warp's lanes in `lanes` as float bits), called
+// by those lanes: one atomic, which nothing waits for.
+__device__ __forceinline__ void raise_max(unsigned* slot, float value, unsigned lanes)
 {
-    const unsigned active = __activemask();
-    const unsigned bits = __reduce_max_sync(active, __float_as_uint(fabsf(value)));
+    const unsigned bits = __reduce_max_sync(lanes, __float_as_uint(fabsf(value)));
     unsigned lane;
     asm("mov.u32 %0, %%laneid;" : "=r"(lane));
-    if (bits && lane == (unsigned)__ffs(active) - 1u) atomicMax(slot, bits);
+    if (bits && lane == (unsigned)__ffs(lanes) - 1u) atomicMax(slot, bits);
 }
+
 // ---- ray blocks ---------------------------------------------------------------------------
 
 // Rays are launched in blocks of 32 (u) x 4 (v).  A CTA's block comes from a

@@ -621,6 +621,7 @@ __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __
         if (lane == 0 && c) atomicAdd(reinterpret_cast<unsigned long long*>(out), c);
         return;
     }
+    const unsigned lanes = __ballot_sync(0xffffffffu, valid);  // (of use to raise_max)
     if (!valid) return;
     if constexpr (!COUNTING) {
         const size_t base = (size_t)(view - view0) * G.Nu * G.Nv;
@@ -650,7 +651,7 @@ __device__ __forceinline__ void column_kernel_body(ExactGeom G, const float4* __
                 const size_t pix = LAYOUT == kLayoutColumns ? base + (size_t)u * G.Nv + row : base + (size_t)row * G.Nu + u;
                 const float x = value(row, acc);
                 store_val<OT>(out + pix, x);
-                if (MODE == 1 && LAYOUT == kLayoutColumns && vmax) raise_max(vmax + view, as_stored<OT>(x));
+                if (MODE == 1 && LAYOUT == kLayoutColumns && vmax) raise_max(vmax + view, as_stored<OT>(x), lanes);
             };
             emit(v, sum.x);
             if (MIRROR) emit(G.Nv - 1 - v, sum.y);
@@ -971,11 +972,10 @@ __global__ void __launch_bounds__(256) column_finish_kernel(ExactGeom G, const f
                 const float ratio = (hf != 0.0f) ? __fdiv_rn(tile[threadIdx.x][threadIdx.y + 8 * q], hf) : 0.0f;
                 val[q] = MODE == 1 ? ratio * w : ratio;
             }
-            if (LAYOUT == kLayoutColumns) {
-                store_val<OT>(out + base + pc, val[q]);
-                if (MODE == 1 && vmax) raise_max(vmax + blockIdx.z, as_stored<OT>(val[q]));
-            }
+            if (LAYOUT == kLayoutColumns) store_val<OT>(out + base + pc, val[q]);
         }
+        // (0 for the lanes beyond the detector)
+        if (LAYOUT == kLayoutColumns && MODE == 1 && vmax) raise_max(vmax + blockIdx.z, as_stored<OT>(val[q]), 0xffffffffu);
     }
     if (LAYOUT == kLayoutRows) {
         __syncthreads();  // the g tile is read
