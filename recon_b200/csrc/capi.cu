@@ -457,8 +457,8 @@ recon_status_t recon_bp_view(recon_plan_t P, const float* d_img, float angle, fl
     cudaStream_t s = as_stream(stream);
     const int vw = view_of_angle(*P, angle);
     if (P->opt.arith == RECON_ARITH_COMPAT) {
-        if (vw >= 0) return compat_bp_view(*P, d_img, (unsigned)vw, false, 0.0f, d_vol, false, s);
-        return compat_bp_view(*P, d_img, 0, true, angle, d_vol, false, s);
+        if (vw >= 0) return compat_bp_view(*P, d_img, (unsigned)vw, false, 0.0f, d_vol, s);
+        return compat_bp_view(*P, d_img, 0, true, angle, d_vol, s);
     }
     if (vw >= 0) return exact_bp(*P, d_img, false, false, (unsigned)vw, 1, false, false, d_vol, nullptr, nullptr, s);
     RB_CHECK(exact_view_table(*P, angle, s));

@@ -897,13 +897,13 @@ static recon_status_t compat_bp_into(Plan& P, const float* img, unsigned view, f
 }
 
 recon_status_t compat_bp_view(Plan& P, const float* img, unsigned view, bool scratch_slot, float angle_scratch,
-                              float* out, bool accumulate, cudaStream_t s)
+                              float* out, cudaStream_t s)
 {
     if (scratch_slot) {
         RB_CHECK(compat_view_loopN(P, angle_scratch, P.nviews, s));
         view = P.nviews;
     }
-    return compat_bp_into(P, img, view, out, accumulate, s);
+    return compat_bp_into(P, img, view, out, false, s);
 }
 
 // Back projections of every plan view (view n's image at img + n * img_stride) summed in

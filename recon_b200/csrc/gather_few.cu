@@ -4,7 +4,9 @@
 // view a warp sets up one, and its chain of dependent loads (view, table, value, image) is
 // all it does.  Here a warp owns eight columns along x: its lanes set them up (four sets of
 // a view and a detector column at a time), the warp then gathers column after column, and
-// the eight are staged so that the image is written in whole sectors.  Lengths, values and order are bp_gather_pairs_kernel's.
+// the eight are staged so that the image is written in whole sectors.  Lengths and values
+// are bp_gather_pairs_kernel's, and so is the order where a voxel has one candidate row per
+// detector column and view; that kernel sums further candidates apart, this one in place.
 //
 // Bound by the latency of a warp's columns, one after the other (a load from L2 each).
 // 256^3 / 512^2, one view: see few_views_suit for both sides.

@@ -35,6 +35,7 @@ namespace exact {
 // A CTA owns TX x TY base columns (kWarps warps) and a loading warp; a stage holds
 // the four views' values of one base view, [r][detector column][row pair].
 constexpr int kStageBytes = 98304;  // a stage: two or four base views of four regions of 12 or 6 KiB
+constexpr unsigned kStages = 2;     // what a block's shared memory holds
 
 template <int EPI, class ST, int PS, int RB, bool SET>
 __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
@@ -46,10 +47,9 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
     constexpr unsigned kPair = 2 * sizeof(ST);  // bytes of a pair
     constexpr int NE = 8 * PS * 32;  // epilogue entries per warp
     constexpr int VB = kStageBytes / (4 * RB);  // base views per stage
-    constexpr int kMaxStages = 4;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ unsigned long long full[kMaxStages], empty[kMaxStages];
-    __shared__ int stage_u[kMaxStages * VB], first_u[32];
+    __shared__ unsigned long long full[kStages], empty[kStages];
+    __shared__ int stage_u[kStages * VB], first_u[32];
     __shared__ StagedItem items[kStagedWarps][32];
     unsigned char* const smem0 = smem + ((128u - (smem_addr(smem) & 127u)) & 127u);
     float4* const szq = reinterpret_cast<float4*>(smem0);  // z planes of the staged rows, as in bp_gather_kernel
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
     const unsigned nitem = SET ? 4u * mc : nview;
     auto view_of = [&](unsigned it) { return SET ? m0 + it % mc + (it / mc) * Q : it; };
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S.stages; ++s) {
+        for (unsigned s = 0; s < kStages; ++s) {
             mbar_init(smem_addr(&full[s]), 1u);
             mbar_init(smem_addr(&empty[s]), nactive);
         }
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
         if (warp == kStagedWarps) {
             // the loading warp: VB items' detector columns into each stage, in turn
             const unsigned bytes = 4u * (unsigned)(S.rows * S.cols) * kPair;
-            unsigned st = base % (unsigned)S.stages, ph = (base / (unsigned)S.stages) & 1u;
+            unsigned st = base % kStages, ph = (base / kStages) & 1u;
             for (unsigned n = 0; n < nuse && ok; ++n) {
                 const unsigned i0 = n * VB, cnt = min((unsigned)VB, nitem - i0);
                 if (i0 % 32u == 0u) {  // 32 items' first detector columns, one per lane
@@ -140,12 +140,12 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
                 }
                 if (!ok) {  // a warp does not answer: let the copies in flight land, then stop
                     if (lane == 0) report_give_up(give_up);
-                    for (unsigned b = 1; b <= min(n, (unsigned)S.stages); ++b) {
+                    for (unsigned b = 1; b <= min(n, kStages); ++b) {
                         const unsigned use = base + n - b;
-                        mbar_wait(smem_addr(&full[use % (unsigned)S.stages]), (use / (unsigned)S.stages) & 1u);
+                        mbar_wait(smem_addr(&full[use % kStages]), (use / kStages) & 1u);
                     }
                 }
-                if (++st == (unsigned)S.stages) {
+                if (++st == kStages) {
                     st = 0;
                     ph ^= 1u;
                 }
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
             };
             const int wshift = __ffs(S.wide) - 1;
             const int per = 32 / S.wide;  // views whose items a warp sets up at a time
-            unsigned st = base % (unsigned)S.stages, ph = (base / (unsigned)S.stages) & 1u;
+            unsigned st = base % kStages, ph = (base / kStages) & 1u;
             for (unsigned vb = 0; vb < nitem; vb += per) {
                 const unsigned nb = min((unsigned)per, nitem - vb);
                 bool valid = false;
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) bp_staged_quarter_kernel(
                     }
                     __syncwarp();  // the stage is read
                     if (lane == 0) mbar_arrive(smem_addr(&empty[st]));
-                    if (++st == (unsigned)S.stages) {
+                    if (++st == kStages) {
                         st = 0;
                         ph ^= 1u;
                     }
@@ -364,12 +364,12 @@ int staged_wide(const Plan& P)
     return rad < 0.9 * (double)E.Rf ? staged_span(P, std::hypot(vx, vy), rad) : 0;
 }
 
-// The boxes that tiles read in chunks of 32 * slots of Zs slices, of a detector whose
-// columns have entries 0 .. top (in multiples of `align` entries): S->wide, cols and rows.
+// The boxes that tiles read in chunks of 32 * slots slices of the lower half, of detector
+// columns in row pairs 0 .. Nv/2 (in multiples of four pairs): S->wide, cols and rows.
 // False where no staged gather serves: a detector too large for staged_item's bounds, a
 // volume that comes near the source (a piece could then lie behind it), a voxel column that
 // meets more than eight detector columns, or a box of more than 256 a side.
-bool staged_boxes(const Plan& P, int slots, int Zs, int top, int align, exact::StagedShape* S)
+static bool staged_boxes(const Plan& P, int slots, exact::StagedShape* S)
 {
     const ExactGeom& E = P.eg;
     if (!staged_bounds_hold(P)) return false;
@@ -382,6 +382,8 @@ bool staged_boxes(const Plan& P, int slots, int Zs, int top, int align, exact::S
     if (wide > 8) return false;
     S->wide = wide <= 1 ? 1 : wide <= 2 ? 2 : wide <= 4 ? 4 : 8;
     S->cols = staged_span(P, std::hypot(tx, ty), rad);
+    constexpr int align = 4;
+    const int Zs = E.Z / 2, top = E.Nv / 2;
     int rows = align;
     for (int k0 = 0; k0 < Zs; k0 += 32 * slots) {
         const double zb = E.P0[2] + k0 * vz, zt = E.P0[2] + std::min(k0 + 32 * slots, Zs) * vz;
@@ -405,17 +407,17 @@ static bool staged_shape(const Plan& P, int slots, size_t value_bytes, exact::St
                          size_t* smem)
 {
     exact::StagedShape S{};
-    if (!staged_boxes(P, slots, P.eg.Z / 2, P.eg.Nv / 2, 4, &S)) return false;
+    if (!staged_boxes(P, slots, &S)) return false;
     const size_t used = (size_t)S.cols * S.rows * 2 * value_bytes;
     if (used > 12288) return false;
     *region = used <= 6144 ? 6144 : 12288;
     const size_t planes = ((size_t)S.rows * sizeof(float4) + 127) / 128 * 128;
     const size_t epilogue = sizeof(float) * exact::kStagedWarps * 8 * slots * 32;
     const size_t room = kStagedSmem - planes;
-    if (2 * (size_t)exact::kStageBytes > room || epilogue > room) return false;
-    S.stages = (int)std::min<size_t>(4, room / exact::kStageBytes);
+    const size_t stages = (size_t)exact::kStages * exact::kStageBytes;
+    if (stages > room || epilogue > room) return false;
     *out = S;
-    *smem = 128 + planes + std::max((size_t)S.stages * exact::kStageBytes, epilogue);  // 128: the base's alignment
+    *smem = 128 + planes + std::max(stages, epilogue);  // 128: the base's alignment
     return true;
 }
 
@@ -433,20 +435,17 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     return fn;
 }
 
-// A table of `table_rows` detector columns of `pitch` entries (a row pair, or a value; an
-// entry is moved as one element of `entry` bytes), read in boxes of S.rows entries x S.cols
-// detector columns.
-bool column_map(const exact::StagedShape& S, const void* vals, size_t pitch, size_t entry, size_t table_rows,
-                CUtensorMap* map)
+// A table of `table_rows` detector columns of `pitch` row pairs (moved as one element of
+// `pair` bytes), read in boxes of S.rows pairs x S.cols detector columns.
+static bool column_map(const exact::StagedShape& S, const void* vals, size_t pitch, size_t pair, size_t table_rows,
+                       CUtensorMap* map)
 {
     const auto encode = tensor_map_encoder();
-    if (!encode || reinterpret_cast<uintptr_t>(vals) % 16 != 0 || pitch * entry % 16 != 0) return false;
+    if (!encode || reinterpret_cast<uintptr_t>(vals) % 16 != 0 || pitch * pair % 16 != 0) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)table_rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)(pitch * entry)};
+    const cuuint64_t strides[1] = {(cuuint64_t)(pitch * pair)};
     const cuuint32_t box[2] = {(cuuint32_t)S.rows, (cuuint32_t)S.cols}, step[2] = {1, 1};
-    const CUtensorMapDataType type = entry == 8   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
-                                     : entry == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32
-                                                  : CU_TENSOR_MAP_DATA_TYPE_UINT16;
+    const CUtensorMapDataType type = pair == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_UINT32;
     return encode(map, type, 2, const_cast<void*>(vals), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;

@@ -1,6 +1,6 @@
-// gather_staged.cuh -- what the staged gather back projectors share: the tile of voxel
-// columns a CTA owns, its loads by TMA and their barriers, the detector columns and rows
-// it needs, and the host side of the boxes (gather_staged.cu, gather_fixed.cu).
+// gather_staged.cuh -- what the staged gather (gather_staged.cu) and the few-view one
+// (gather_few.cu) share, and the staged one's tile of voxel columns, its loads by TMA and
+// their barriers, and the detector columns and rows it needs.
 #pragma once
 
 #include "gather_device.cuh"
@@ -17,9 +17,8 @@ constexpr int kStagedThreads = (kStagedWarps + 1) * 32;
 
 // What a stage holds and how columns meet the detector, from the host (staged_shape).
 struct StagedShape {
-    int rows;     // staged entries per detector column (multiple of 4): the box's width
+    int rows;     // staged row pairs per detector column (multiple of 4): the box's width
     int cols;     // staged detector columns per view: the box's height
-    int stages;   // stages in flight
     int wide;     // most detector columns one voxel column meets in a view: 1, 2, 4 or 8
 };
 
@@ -116,8 +115,8 @@ __device__ __forceinline__ float4 lds_planes(unsigned a)
     return p;
 }
 
-// Sum of |a| d / ... : the rows (relative to row 0) that heights [zb, zt] can be
-// seen at from depths [dmin, dmax], widened by one row.
+// The rows that heights [zb, zt] are seen at from depths [dmin, dmax], widened by one row on
+// either side.
 __device__ __forceinline__ void staged_rows(const GatherConst& C, float zb, float zt, float dmin, float dmax,
                                             float& lo, float& hi)
 {
@@ -188,8 +187,5 @@ __device__ __forceinline__ bool staged_item(const ExactGeom& G, const GatherCons
 constexpr size_t kStagedSmem = 227 * 1024 - sizeof(exact::StagedItem) * 32 * exact::kStagedWarps - 1536;
 
 int staged_wide(const Plan& P);
-bool staged_boxes(const Plan& P, int slots, int Zs, int top, int align, exact::StagedShape* S);
-bool column_map(const exact::StagedShape& S, const void* vals, size_t pitch, size_t entry, size_t table_rows,
-                CUtensorMap* map);
 
 }  // namespace rb

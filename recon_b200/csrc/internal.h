@@ -255,8 +255,7 @@ recon_status_t exact_bp(Plan& P, const void* sino, bool sino_is_rw, bool bf16, u
 recon_status_t compat_fp(Plan& P, const float* vol, unsigned first, unsigned count, bool scratch_slot,
                          float angle_scratch, float* out, cudaStream_t s);
 recon_status_t compat_bp_view(Plan& P, const float* img, unsigned view, bool scratch_slot,
-                              float angle_scratch, float* out_or_accum, bool accumulate,
-                              cudaStream_t s);
+                              float angle_scratch, float* out, cudaStream_t s);
 recon_status_t compat_alloc_volume(Plan& P);
 recon_status_t compat_bp_views(Plan& P, const float* sino, unsigned first, unsigned count, float* out, cudaStream_t s);
 // vol[z][y][x] -> out[(y*X + x)*(Z + 2*pad) + z + pad] (fpcol.cu); the padding is not written

@@ -82,5 +82,5 @@ extern "C" recon_status_t recon_compat_bp_view_noalloc(const recon_geometry_t* g
     // (the angle, loopN and maxabs slots and the accumulator are written or cleared by the
     // projector itself)
     // view slot 0 (= P.nviews): angle and step count set up for this call
-    return compat_bp_view(P, d_img, 0, true, angle_deg, d_vol, false, s);
+    return compat_bp_view(P, d_img, 0, true, angle_deg, d_vol, s);
 }
