@@ -3,8 +3,11 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "internal.h"
 
@@ -29,6 +32,57 @@ recon_status_t cuda_fail(cudaError_t e, const char* what)
     return fail(e == cudaErrorMemoryAllocation ? RECON_ERR_OUT_OF_MEMORY : RECON_ERR_CUDA, m);
 }
 
+// Words of host memory that kernels write (Plan::h_give_up): a page of them is registered
+// when the first plan needs one and kept, because a page of its own would cost each plan 1.3
+// to 2.8 ms (1.5 ms is all that a 128^3 plan takes).  Another page follows only where all
+// words are taken.
+namespace {
+constexpr size_t kGiveUpWords = 1024;
+struct GiveUpPage {
+    unsigned* words;
+    std::vector<bool> taken;
+};
+std::mutex g_give_up_mutex;
+std::vector<GiveUpPage> g_give_up_pages;
+}  // namespace
+
+static recon_status_t take_give_up_word(Plan& P)
+{
+    std::lock_guard<std::mutex> lock(g_give_up_mutex);
+    size_t n = 0, w = kGiveUpWords;
+    for (; n < g_give_up_pages.size(); ++n) {
+        const auto& t = g_give_up_pages[n].taken;
+        w = (size_t)(std::find(t.begin(), t.end(), false) - t.begin());
+        if (w < kGiveUpWords) break;
+    }
+    if (n == g_give_up_pages.size()) {
+        void* p = nullptr;
+        if (posix_memalign(&p, 4096, kGiveUpWords * sizeof(unsigned)) != 0)
+            return fail(RECON_ERR_OUT_OF_MEMORY, "no host memory");
+        g_give_up_pages.push_back({static_cast<unsigned*>(p), std::vector<bool>(kGiveUpWords, false)});
+        w = 0;
+    }
+    GiveUpPage& page = g_give_up_pages[n];
+    unsigned* d = nullptr;
+    if (cudaHostGetDevicePointer((void**)&d, page.words, 0) != cudaSuccess) {  // new, or the device was reset
+        cudaGetLastError();
+        RB_CUDA(cudaHostRegister(page.words, kGiveUpWords * sizeof(unsigned), cudaHostRegisterMapped | cudaHostRegisterPortable));
+        RB_CUDA(cudaHostGetDevicePointer((void**)&d, page.words, 0));
+    }
+    page.taken[w] = true;
+    page.words[w] = 0u;
+    P.h_give_up = page.words + w;
+    P.d_give_up = d + w;
+    return RECON_OK;
+}
+
+static void release_give_up_word(unsigned* word)
+{
+    std::lock_guard<std::mutex> lock(g_give_up_mutex);
+    for (GiveUpPage& page : g_give_up_pages)
+        if (word >= page.words && word < page.words + kGiveUpWords) page.taken[word - page.words] = false;
+}
+
 Plan::~Plan()
 {
     int cur = -1;
@@ -37,7 +91,7 @@ Plan::~Plan()
     release_plan_textures(this);
     if (vol_z_free) cudaEventDestroy(vol_z_free);
     for (void* p : allocations) cudaFree(p);
-    if (h_give_up) cudaFreeHost(h_give_up);
+    if (h_give_up) release_give_up_word(h_give_up);
     if (cur >= 0 && cur != device) cudaSetDevice(cur);
 }
 
@@ -328,11 +382,7 @@ recon_status_t recon_plan_create(const recon_geometry_t* geom, const recon_optio
             const bool gather = P->bp_gather && !tuned;
             if (gather || tuned) {
                 exact_use_gather(*P, true);
-                if (P->quarter) {  // the staged gather waits for its copies
-                    RB_CUDA(cudaHostAlloc((void**)&P->h_give_up, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable));
-                    *P->h_give_up = 0u;
-                    RB_CUDA(cudaHostGetDevicePointer((void**)&P->d_give_up, P->h_give_up, 0));
-                }
+                if (P->quarter) RB_CHECK(take_give_up_word(*P));  // the staged gather waits for its copies
                 if (P->col_pairs) RB_CHECK(build_wq_pairs(*P));
             }
             if (!gather) {

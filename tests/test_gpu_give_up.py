@@ -47,3 +47,17 @@ def test_other_plans_have_no_waits():
         _run_out(P)
     assert err.value.status == RECON_ERR_UNSUPPORTED
     P.check()
+
+
+def test_each_plan_has_its_own_report():
+    plans = [Plan(CFG, Options(siddon_bp=SIDDON_BP_GATHER)) for _ in range(3)]
+    _run_out(plans[1])
+    plans[0].check()
+    plans[2].check()
+    with pytest.raises(ReconError, match="ran out"):
+        plans[1].check()
+    _run_out(plans[1])
+    plans[1].close()  # its word goes to the next plan, cleared
+    again = Plan(CFG, Options(siddon_bp=SIDDON_BP_GATHER))
+    for P in (plans[0], plans[2], again):
+        P.check()
