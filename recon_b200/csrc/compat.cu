@@ -371,10 +371,10 @@ __device__ __forceinline__ void walk(const CompatGeom& G, const Ray& r, unsigned
     part(r.amax, cur);
 }
 
-// Bound by instruction issue (85 % of peak).  256^3 / 360 views / 512^2: forward 19.2 ->
+// Bound by instruction issue (83 % of peak).  256^3 / 360 views / 512^2: forward 19.2 ->
 // 13.5 ms and scatter 19.4 -> 14.1 ms, from lanes along detector columns that branched
 // apart at every step, in a grid that had every view's rays cross an accumulator larger
-// than L2 (40 GB of DRAM traffic per scatter).
+// than L2 (41 GB of DRAM traffic per scatter, now 0.8 GB).
 // Rays of a CTA: 32 detector rows (lanes) x 8 detector columns.  The rays of one
 // detector column cross nearly the same (x, y) voxel columns, so a warp's lanes step
 // alike, and their voxels lie next to each other in an image whose z runs fastest.

@@ -694,11 +694,11 @@ constexpr auto fp_column_kernel_of()
 // times it, rounded to an integer, to the 64-bit accumulator of the voxel it crosses (z
 // fastest, a layer of padding at each end that takes what lies outside): the products and
 // the sums of bp_ray_kernel (exact.cu) bit for bit, as integer sums do not depend on the
-// order.  The rows of a warp add to neighbouring addresses: about 10 sectors of L2 per warp
-// reduction against the slabs' 17, no slab walked twice, and the path found once for all
-// rows.  Bound by L2's atomics (61 % of its throughput at 200 x 200 x 120, 0.9e12 products
-// a second).  Per back projection, slabs to columns: 200 x 200 x 120 / 240 views in eight
-// subsets 2.83 -> 2.28 ms, 208^3 / 200 views 2.93 -> 1.64, 131 x 117 x 93 / 77 views 0.210 ->
+// order.  The rows of a warp add to neighbouring addresses: 11.8 sectors of L2 per warp
+// reduction against the slabs' 21.4, no slab walked twice, and the path found once for all
+// rows.  Bound by L2's atomics (70 % of its throughput, 0.51e12 products a second, from 240
+// views of 384 x 256 without a zero onto 200 x 200 x 120).  Per back projection, slabs to
+// columns: the same 240 views of a phantom's ratio in eight subsets 2.83 -> 2.28 ms, 208^3 / 200 views 2.93 -> 1.64, 131 x 117 x 93 / 77 views 0.210 ->
 // 0.134.  (A gather of the same integers from values staged in shared memory won 1.3 to
 // 1.6 times where rows mirror and lie a voxel apart and lost elsewhere.)
 

@@ -11,13 +11,12 @@
 //
 // Measured (256^3, 360 views, 512^2; one B200): 1.56 ms against
 // bp_gather_quarter_kernel's 2.41 ms; 512^3, 720 views, 1024 x 768, BF16 ratio:
-// 22.8 against 40.2 ms.  Bound by shared-memory reads (about 80 % of their
-// wavefront peak: 52 wavefronts for the 1024 products of one detector column) with
-// 0.94e9 warp instructions (1.56e9).  What brought it there: loading the columns one
-// by one with untiled bulk copies 3.46 ms (28 copies a view, the loading warp the
-// limit), TMA boxes 2.10, two or four views to a stage instead of one 1.75, packed
-// multiply-adds without a predicate 1.56.  Reading the zero entry of a region in place
-// of the predicate cost bank conflicts (2.05).
+// 22.8 against 40.2 ms.  Bound by shared-memory reads (77 % of the wavefront peak:
+// 0.34e9 wavefronts, 68 for 1024 products) with 0.94e9 warp instructions (1.56e9).
+// What brought it there: loading the columns one by one with untiled bulk copies 3.46 ms
+// (28 copies a view, the loading warp the limit), TMA boxes 2.10, two or four views to a
+// stage instead of one 1.75, packed multiply-adds without a predicate 1.56.  Reading the
+// zero entry of a region in place of the predicate cost bank conflicts (2.05).
 #include "gather_staged.cuh"
 
 #include <algorithm>
