@@ -691,6 +691,7 @@ __global__ void max_views_kernel(const unsigned* __restrict__ maxabs, unsigned n
 // at 256^3 / 512^2 four views take 270 us without and 281 us with it, eight 458 and
 // 436, sixteen 856 and 744 (64^3 and 128^3: within 3 us of each other from three on).
 constexpr unsigned kZfastViews = 6;
+constexpr int kZfastSlices = 32 * 65535;  // and most slices (launch_zfast's grid)
 
 static dim3 ray_block() { return dim3(32, 4, 1); }
 static dim3 ray_grid(const Plan& P, unsigned views)
@@ -728,8 +729,9 @@ static recon_status_t launch_compat_fp(Plan& P, unsigned first, unsigned count, 
                                        float* out, unsigned* maxabs, float* scratch, cudaStream_t s)
 {
     if (count == 0) return RECON_OK;
-    float* copy = count >= kZfastViews ? scratch : nullptr;
-    const bool shared = count >= kZfastViews && !scratch && P.d_vol_z;
+    const bool wanted = count >= kZfastViews && P.cg.dims[2] <= kZfastSlices;
+    float* copy = wanted ? scratch : nullptr;
+    const bool shared = wanted && !scratch && P.d_vol_z;
     if (shared) {
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         RB_CUDA(cudaStreamIsCapturing(s, &capturing));
@@ -753,7 +755,7 @@ static recon_status_t launch_compat_fp(Plan& P, unsigned first, unsigned count, 
 // get it projects from the caller's volume.
 recon_status_t compat_alloc_volume(Plan& P)
 {
-    if (P.nviews < kZfastViews) return RECON_OK;
+    if (P.nviews < kZfastViews || P.cg.dims[2] > kZfastSlices) return RECON_OK;
     if (P.alloc(&P.d_vol_z, P.nvox, "z-fastest volume") != RECON_OK) {
         P.d_vol_z = nullptr;
         return RECON_OK;
