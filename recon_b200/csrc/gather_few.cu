@@ -156,14 +156,27 @@ static size_t few_smem(const Plan& P, unsigned count, int wide)
            exact::kFewWarps * (sets * exact::kFewStage * sizeof(exact::StagedItem) + (sets + 3) / 4 * sizeof(unsigned));
 }
 
-// The few-view kernel serves one or two views on mirrored row pairs, and up to four where
-// there are 16384 columns to share its warps' latency.  Against bp_gather_pairs_kernel, us
-// for one and four views, layout included: 64^3 16.8 and 22.9 against 16.7 and 16.1; 128^3
-// 16.4 and 27 against 23 and 29; 256^3 46 and 96 against 82 and 117; 512^3 267 and 607
-// against 560 and 801; six views 131 against 138 at 256^3, 36 against 34 at 128^3.
+// The few-view kernel's side of the line against bp_gather_pairs_kernel: enough columns
+// (x, y) to share its warps' latency.  us with and without it, layout included; rows a voxel
+// apart (AUTO's gather): 80^3 one view 15 and 14, 96^3 one 15 and 17, two 17 and 17, 96 x 96
+// x 300 22 and 26, 27 and 29, 48 x 48 x 300 21 and 14, 25 and 15; 128^3 one to four 15 19 23 28
+// and 23 25 27 30; 256^3 47 58 73 98 and 82 95 107 119.  Closer rows, of which voxels have
+// several: 96^3 one 19 and 20, 96 x 96 x 160 23 and 21, 112^3 21 and 23, 112 x 112 x 300 38 and 39; two views
+// 128^3 29 and 33, 160^3 62 and 56 (800 CTAs, a round and a third), 200^3 80 and 88, 256^3 130
+// and 146; three 128^3 43 and 39, 256^3 194 and 183 (but 200 x 200 x 64 49 and 64, four 62 and
+// 74: up to 64 slices the same line as for rows a voxel apart).
 static int few_views_suit(const Plan& P, unsigned count)
 {
-    if (!P.col_pairs || count == 0 || count > 4 || (count > 2 && (size_t)P.eg.X * P.eg.Y < 16384)) return 0;
+    const ExactGeom& E = P.eg;
+    const size_t columns = (size_t)E.X * E.Y;
+    if (!P.col_pairs || count == 0 || count > 4) return 0;
+    if (E.Z > 64 && several_candidate_rows(P)) {
+        const int ctas = ((E.X + exact::kFewStage - 1) / exact::kFewStage) * ((E.Y + exact::kFewWarps - 1) / exact::kFewWarps);
+        if (count > 2 || columns < (E.Z <= 128 ? 9216u : 12544u)) return 0;
+        if (count == 2 && (columns < 16384 || (ctas > 4 * P.sm_count && ctas < 8 * P.sm_count))) return 0;
+    } else if (columns < (count <= 2 ? 9216u : 16384u)) {
+        return 0;
+    }
     const int wide = staged_wide(P);
     return wide > 0 && wide <= 4 && few_smem(P, count, wide) <= kFewSmem ? wide : 0;
 }

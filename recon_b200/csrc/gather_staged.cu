@@ -351,6 +351,16 @@ static int staged_span(const Plan& P, double d, double rad)
 // of up to Nu, 0.007 column at 8192.  (Exact division would give 0.0012 and 0.005.)
 static bool staged_bounds_hold(const Plan& P) { return P.eg.Nv <= 4096 && P.eg.Nu <= 8192; }
 
+// Voxels meet clearly more than one detector row per detector column and view: the rows'
+// distance and the slant of a voxel column's piece, where both are largest.
+bool several_candidate_rows(const Plan& P)
+{
+    const ExactGeom& E = P.eg;
+    const double vx = E.vox[0], vy = E.vox[1], vz = E.vox[2], ez = std::fabs((double)E.Ry / E.dv);
+    const double near = (double)E.Rf - 0.5 * std::hypot(E.X * vx, E.Y * vy);
+    return !(near > 0.0) || (vz + 0.5 * E.Z * vz * std::hypot(vx, vy) / near) * ez / near > 1.05;
+}
+
 // Most detector columns that one voxel column meets in a view, or 0 where staged_item does
 // not serve: its bounds do not hold, or the volume comes near the source (where a piece
 // could lie behind it).
@@ -490,7 +500,14 @@ recon_status_t staged_quarter_gather(Plan& P, const ST* vals, size_t view_stride
     // view_stride 0: the same table for every view (the weights of the sensitivity)
     const unsigned view_rows = view_stride ? (unsigned)P.eg.Nu : 0u;
     const size_t table_rows = view_stride ? (size_t)P.eg.Nu * P.nviews : (size_t)P.eg.Nu;
-    *served = P.d_give_up && table_rows < 0x7fffffff && staged_shape(P, slots, sizeof(ST), &S, &region, &smem) &&
+    // Fewer tiles than half the SMs: bp_gather_quarter_kernel, whose tiles are half as large, is
+    // as fast or faster at the weights (one table for every view: 64 x 64 x 300, 80 views, 88
+    // against 92 us, 64 x 64 x 512 103 / 113) and, where voxels have several candidate rows, at
+    // volumes of two chunks (48 x 48 x 300 293 / 305, 64 x 64 x 512 424 / 451).
+    const int H = P.eg.X / 2, tiles = (H + exact::kStagedTX - 1) / exact::kStagedTX * ((H + exact::kStagedTY - 1) / exact::kStagedTY);
+    const bool few_tiles = 2 * tiles <= P.sm_count &&
+                           (EPI == 0 && view_stride == 0 ? P.eg.Z > 128 : P.eg.Z > 256 && several_candidate_rows(P));
+    *served = P.d_give_up && !few_tiles && table_rows < 0x7fffffff && staged_shape(P, slots, sizeof(ST), &S, &region, &smem) &&
               column_map(S, vals, pair_entries(P.eg.Nv), 2 * sizeof(ST), table_rows, &map);
     if (!*served) return RECON_OK;
     auto run = [&](auto ps) -> recon_status_t {

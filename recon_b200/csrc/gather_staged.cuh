@@ -187,5 +187,6 @@ __device__ __forceinline__ bool staged_item(const ExactGeom& G, const GatherCons
 constexpr size_t kStagedSmem = 227 * 1024 - sizeof(exact::StagedItem) * 32 * exact::kStagedWarps - 1536;
 
 int staged_wide(const Plan& P);
+bool several_candidate_rows(const Plan& P);
 
 }  // namespace rb

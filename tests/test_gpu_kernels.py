@@ -12,7 +12,6 @@ if not torch.cuda.is_available():
 
 from recon_b200 import (ARITH_COMPAT, BP_VOXEL, PROJECTOR_BACK, PROJECTOR_FORWARD, SIDDON_BP_GATHER,  # noqa: E402
                         SIDDON_BP_RAY, SUM_PLAIN, Options, Plan)
-from test_gpu_few_views import GEOMS as FEW  # noqa: E402
 from test_gpu_fp_wide import BIG  # noqa: E402
 from test_gpu_ray_columns import GEOMS as RAY  # noqa: E402
 from test_gpu_staged import QUARTER  # noqa: E402
@@ -42,6 +41,9 @@ def test_quarter_turns(name):
     assert back(P) == "bp_staged_quarter_kernel"
     assert iteration(P)[1] == "bp_staged_quarter_kernel"
     assert back(P, 3) != "bp_staged_quarter_kernel"
+    P.sensitivity()  # (few tiles of a tall volume: the smaller ones of the other kernel)
+    tall = QUARTER[name]["Zdim"] > 128
+    assert P.last_kernel(PROJECTOR_BACK) == ("bp_gather_quarter_kernel" if tall else "bp_staged_quarter_kernel")
     P.mlem_forward_quarters(P.new_sinogram(), P.new_volume(1.0), 0, 1)
     P.mlem_backward_quarters(P.new_volume(), 0, 1)
     assert P.last_kernel(PROJECTOR_BACK) == "bp_staged_quarter_kernel"
@@ -56,21 +58,36 @@ def test_quarter_turns_without_stages():
         assert back(P) == "bp_gather_quarter_kernel"
 
 
-@pytest.mark.parametrize("name", list(FEW))
-def test_few_views(name):
-    P = Plan(FEW[name], Options(siddon_bp=SIDDON_BP_GATHER))
-    large = FEW[name]["Xdim"] * FEW[name]["Ydim"] >= 16384
-    assert [back(P, n) for n in (1, 2)] == ["bp_gather_few_kernel"] * 2
-    assert [back(P, n) for n in (3, 4)] == ["bp_gather_few_kernel" if large else "bp_gather_pairs_kernel"] * 2
-    assert back(P, 5) == "bp_gather_pairs_kernel"
+FEW_ROWS = dict(TAxPixels=24, TAxPixDim=3.0)  # rows further apart than voxels: one candidate
+FEW_LINES = {  # columns (x, y): views that take the few-view kernel, with one candidate row, with several
+    (95, 95): ([], []),
+    (96, 96): ([1, 2], []),
+    (112, 112): ([1, 2], [1]),
+    (128, 128): ([1, 2, 3, 4], [1, 2]),
+    (160, 160): ([1, 2, 3, 4], [1]),
+    (200, 200): ([1, 2, 3, 4], [1, 2]),
+}
+
+
+@pytest.mark.parametrize("x, y", list(FEW_LINES))
+@pytest.mark.parametrize("several", [False, True])
+def test_few_views(x, y, several):
+    cfg = small_cfg(Xdim=x, Ydim=y, Zdim=24, XVoxSize=0.25, YVoxSize=0.25, **({} if several else FEW_ROWS))
+    if several:
+        cfg.update(Zdim=130, ZVoxSize=0.25, TAxPixels=150, TAxPixDim=0.3)
+    P = Plan(cfg, Options(siddon_bp=SIDDON_BP_GATHER))
+    few = FEW_LINES[(x, y)][several]
+    for n in range(1, 6):
+        assert back(P, n) == ("bp_gather_few_kernel" if n in few else "bp_gather_pairs_kernel"), n
     P.bp_view(torch.ones((P.nv, P.nu), device="cuda"), 41.5)
-    assert P.last_kernel(PROJECTOR_BACK) == "bp_gather_few_kernel"
+    assert P.last_kernel(PROJECTOR_BACK) == ("bp_gather_few_kernel" if 1 in few else "bp_gather_pairs_kernel")
 
 
 def test_large_detectors():
     """Up to 4096 rows and 8192 columns the few-view gather's bounds hold; it drops no ray there."""
     for rows, columns in ((4096, 64), (4098, 64), (48, 8192), (48, 8193)):
-        cfg = small_cfg(TAxPixels=rows, TAxPixDim=72.0 / rows, AxPixels=columns, AxPixDim=96.0 / min(columns, 96))
+        cfg = small_cfg(Xdim=112, Ydim=112, XVoxSize=0.3, YVoxSize=0.3, TAxPixels=rows, TAxPixDim=72.0 / rows,
+                        AxPixels=columns, AxPixDim=96.0 / min(columns, 96))
         P = Plan(cfg, Options(siddon_bp=SIDDON_BP_GATHER))
         y = torch.rand((1, P.nv, P.nu), device="cuda", generator=torch.Generator("cuda").manual_seed(341))
         out = P.bp_views(y, 3, 1)
