@@ -1770,8 +1770,9 @@ static recon_status_t launch_bp(Plan& P, const ST* sino, unsigned first, unsigne
         dim3 grid;
         const uint2* tiles;
         unsigned n_launch;
-        ray_launch(P, slab < (int)P.bp_tiles.size() ? P.bp_tiles[slab] : none, first, count, &grid, &tiles,
-                   &n_launch);
+        // (a plan that keeps a slab beside the columns has one, of the whole volume)
+        ray_launch(P, P.bp_columns ? P.fp_tiles : slab < (int)P.bp_tiles.size() ? P.bp_tiles[slab] : none, first, count,
+                   &grid, &tiles, &n_launch);
         if (n_launch) {
             exact::bp_ray_kernel<RMODE, WEIGHTED, ST><<<grid, blk, 0, s>>>(P.eg, P.d_txy, P.d_kxy, P.d_cs, P.d_zp,
                                                                            P.d_w, tiles, first, sino, P.d_bpmax,
@@ -1911,12 +1912,10 @@ recon_status_t exact_tune_bp(Plan& P)
         g_bp_tune_gather.emplace(key, gather);
     }
     exact_use_gather(P, gather);
-    if (gather && P.d_bpacc) {
-        const size_t words = P.d_bpacc_t ? (size_t)P.eg.X * P.eg.Y * bp_slab_depth(P) : bp_acc_words(P) + 1;
-        plan_release(P, P.d_bpacc, words * sizeof(unsigned long long));
-        plan_release(P, P.d_bpacc_t, words * sizeof(unsigned long long));
+    if (gather) {
+        plan_release(P, P.d_bpsum, P.bpsum_words * sizeof(unsigned long long));
         plan_release(P, P.d_bpmax, sizeof(unsigned));
-        P.d_bpacc = P.d_bpacc_t = nullptr;
+        P.d_bpsum = P.d_bpcol = P.d_bpacc = P.d_bpacc_t = nullptr;
         P.d_bpmax = nullptr;
     }
     return RECON_OK;
@@ -2213,6 +2212,9 @@ recon_status_t launch_maxabs(Plan& P, const float* sino, unsigned count, unsigne
 // whole volume, z fastest, padded).
 size_t bp_acc_words(const Plan& P) { return (size_t)P.eg.X * P.eg.Y * (P.eg.Z + 2); }
 
+// Words allocated for it: cleared in pairs, and a slab's accumulators follow on 16 bytes.
+static size_t bp_column_words(const Plan& P) { return (bp_acc_words(P) + 1) / 2 * 2; }
+
 // Makes the plan's Siddon back projector the gather or the ray design.  The ray design
 // adds along detector columns (bp_column_kernel, fpcol.cu) wherever the forward projector
 // walks them, with the same sums as ray by ray in slabs (bp_ray_kernel), which is left to
@@ -2226,14 +2228,30 @@ void exact_use_gather(Plan& P, bool gather)
     P.col_pairs = gather && exact_pairs_suit(P);
 }
 
+// A sinogram's back projections of few rays into a small volume are launches more than
+// work, and ray by ray needs nothing cleared first: a call takes the slabs where the volume
+// has at most 2^20 voxels and the call up to four views or 160000 rays.  Slabs against
+// columns, us, for 1, 4, 8 and 32 views: 32^3 / 64^2 17 17 20 30 against 20 22 23 33, 60 views
+// 46 and 43; 64^3 / 128^2 18 19 24 54 against 22 24 28 42 (twelve 35 and 30); 48 x 41 x 51 / 97
+// x 77 17 18 21 41 against 20 21 23 45; 96^3 / 180^2 23 35 53 145 against 25 37 55 145; 48 x 48
+// x 300 / 96 x 500 23 31 46 98 against 27 35 49 83.  A larger volume: 128^3, 1 and 4, 30 45
+// against 29 43.
+static bool few_rays_by_slabs(const Plan& P, unsigned count)
+{
+    return P.d_bpacc && (count <= 4 || P.npix * count <= 160000);
+}
+
 // The ray design's accumulators: the whole volume's (8 bytes a voxel) along detector
-// columns, else two of a slab of at most 64 MiB together.  A device without room for the
+// columns, and a small volume's slab; else two of a slab of at most 64 MiB together.  A device without room for the
 // first and the buffers that an MLEM iteration will add (looked at where the first takes
 // more than the slabs would) gets the second, which give the same bits more slowly.
 recon_status_t exact_alloc_ray(Plan& P)
 {
+    const size_t slab = (size_t)P.eg.X * P.eg.Y * bp_slab_depth(P);
+    size_t column = 0, words = 2 * slab;  // of one allocation, the whole volume's accumulator first
     if (P.bp_columns) {
-        const size_t words = bp_acc_words(P) + 1;  // cleared in pairs
+        column = bp_column_words(P);
+        words = column + (P.nvox <= size_t(1) << 20 ? 2 * slab : 0);
         bool room = true;
         if (words * sizeof(unsigned long long) > size_t(64) << 20) {
             size_t free_bytes = 0, total = 0;
@@ -2243,21 +2261,25 @@ recon_status_t exact_alloc_ray(Plan& P)
             room = words * sizeof(unsigned long long) + iteration <= free_bytes;
         }
         const recon_status_t st =
-            room ? P.alloc(&P.d_bpacc, words, "back projection accumulator") : RECON_ERR_OUT_OF_MEMORY;
+            room ? P.alloc(&P.d_bpsum, words, "back projection accumulator") : RECON_ERR_OUT_OF_MEMORY;
+        if (st != RECON_OK && st != RECON_ERR_OUT_OF_MEMORY) return st;
         if (st == RECON_OK) {
             RB_CHECK(build_view_maxima(P));
-            return P.alloc(&P.d_bpmax, 1, "back projection max");
+        } else {
+            P.bp_no_room = true;
+            exact_use_gather(P, false);
+            column = 0;
+            words = 2 * slab;
         }
-        if (st != RECON_ERR_OUT_OF_MEMORY) return st;
-        P.bp_no_room = true;
-        exact_use_gather(P, false);
     }
-    const size_t slab = (size_t)P.eg.X * P.eg.Y * bp_slab_depth(P);
-    RB_CHECK(P.alloc(&P.d_bpacc, slab, "back projection accumulator"));
-    RB_CHECK(P.alloc(&P.d_bpacc_t, slab, "back projection accumulator (transposed)"));
+    if (!P.d_bpsum) RB_CHECK(P.alloc(&P.d_bpsum, words, "back projection accumulators"));
+    P.bpsum_words = words;
     RB_CHECK(P.alloc(&P.d_bpmax, 1, "back projection max"));
-    RB_CUDA(cudaMemset(P.d_bpacc, 0, slab * sizeof(unsigned long long)));
-    RB_CUDA(cudaMemset(P.d_bpacc_t, 0, slab * sizeof(unsigned long long)));
+    if (column) P.d_bpcol = P.d_bpsum;
+    if (words == column) return RECON_OK;
+    P.d_bpacc = P.d_bpsum + column;
+    P.d_bpacc_t = P.d_bpacc + slab;
+    RB_CUDA(cudaMemset(P.d_bpacc, 0, 2 * slab * sizeof(unsigned long long)));
     return RECON_OK;
 }
 
@@ -2292,6 +2314,7 @@ recon_status_t exact_bp(Plan& P, const void* sino, bool sino_is_rw, bool bf16, u
             return bp_columns<float>(P, (const float*)sino, P.npix, nullptr, first, count, m, count, out, sn, s);
         }
         // a sinogram [view][v][u], read and weighted in place
+        if (few_rays_by_slabs(P, count)) return launch_bp<0, true, float>(P, (const float*)sino, first, count, vol, nullptr, s);
         return bp_columns<float>(P, (const float*)sino, P.npix, P.d_wq, first, count, nullptr, 0u, vol, nullptr, s);
     }
     if (P.bp_gather) {

@@ -1349,7 +1349,11 @@ static recon_status_t launch_bp_column(Plan& P, unsigned first, unsigned count, 
         // a launch of few warps takes the paths in stretches (the sums do not care)
         const double warps = (double)grid.x * grid.y * grid.z * (rows / 32);
         const double most = std::max(1, (E.X + E.Y) / kStretch);  // pieces enough to be worth finding the path
-        const int nseg = (int)std::min({8.0, most, std::max(1.0, 32.0 * P.sm_count / warps)});
+        int nseg = (int)std::min({8.0, most, std::max(1.0, 32.0 * P.sm_count / warps)});
+        // two stretches up to two rounds of the 48 warps an SM holds, where paths are long: us
+        // with one and with two, 128^3, 24 views 138 and 111; 150 x 141 x 133, four 101 and 87;
+        // 200^3, six 250 and 213; 256 x 250 x 244, three 281 and 244
+        if (nseg == 1 && E.X + E.Y >= 160 && warps <= 96.0 * P.sm_count) nseg = 2;
         if (tiles) grid.y *= nseg;
         else grid.z *= nseg;
         kernel<<<grid, rows, smem, s>>>(E, P.d_txy, P.d_kxy, P.d_zp, tiles, first, v0, nseg, vf, vb, view_stride, wq, P.d_bpmax,
@@ -1386,7 +1390,7 @@ recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, const flo
     const int cbits = bp_count_bits(P, count);
     const size_t pairs = (bp_acc_words(P) + 1) / 2;
     const unsigned blocks = (unsigned)std::min<size_t>((pairs + 255) / 256, (size_t)P.sm_count * 16);
-    exact::bp_clear_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<ulonglong2*>(P.d_bpacc), pairs, sino_max ? nullptr : vmax,
+    exact::bp_clear_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<ulonglong2*>(P.d_bpcol), pairs, sino_max ? nullptr : vmax,
                                                   sino_max ? 0u : nmax, P.d_bpmax);
     RB_CUDA(cudaGetLastError());
     if (sino_max) RB_CHECK(launch_maxabs(P, (const float*)vals, count, P.d_bpmax, s));
@@ -1394,12 +1398,12 @@ recon_status_t bp_columns(Plan& P, const ST* vals, size_t view_stride, const flo
     const __nv_bfloat16* vb = nullptr;
     if constexpr (std::is_same<ST, float>::value) vf = vals;
     else vb = vals;
-    RB_CHECK(launch_bp_column<false>(P, first, count, vf, vb, view_stride, wq, max_len, cbits, P.d_bpacc, s));
+    RB_CHECK(launch_bp_column<false>(P, first, count, vf, vb, view_stride, wq, max_len, cbits, P.d_bpcol, s));
     const dim3 fgrid((unsigned)((E.X + 31) / 32) * (unsigned)((E.Z + 31) / 32), std::min(E.Y, 65535));
     if (sens)
-        exact::bp_column_finish_kernel<2><<<fgrid, dim3(32, 8), 0, s>>>(E, P.d_bpmax, max_len, cbits, P.d_bpacc, vol, sens);
+        exact::bp_column_finish_kernel<2><<<fgrid, dim3(32, 8), 0, s>>>(E, P.d_bpmax, max_len, cbits, P.d_bpcol, vol, sens);
     else
-        exact::bp_column_finish_kernel<0><<<fgrid, dim3(32, 8), 0, s>>>(E, P.d_bpmax, max_len, cbits, P.d_bpacc, vol, sens);
+        exact::bp_column_finish_kernel<0><<<fgrid, dim3(32, 8), 0, s>>>(E, P.d_bpmax, max_len, cbits, P.d_bpcol, vol, sens);
     RB_CUDA(cudaGetLastError());
     return RECON_OK;
 }

@@ -150,7 +150,10 @@ struct Plan {
     cudaEvent_t vol_z_free = nullptr;  // COMPAT: the last use of d_vol_z (by calls outside stream captures)
     // back projection: fixed-point accumulators of one z-slab, image layout
     // and xy-transposed, and the max |value| of the call's input (float bits)
-    unsigned long long* d_bpacc = nullptr;
+    unsigned long long* d_bpsum = nullptr;  // what holds the next three
+    size_t bpsum_words = 0;
+    unsigned long long* d_bpcol = nullptr;  // bp_columns: accumulator of the whole volume, z fastest, padded
+    unsigned long long* d_bpacc = nullptr;  // slabs (bp_columns: small volumes' calls of few rays)
     unsigned long long* d_bpacc_t = nullptr;
     unsigned* d_bpmax = nullptr;
     // ray blocks crossing the volume (forward projection) and each

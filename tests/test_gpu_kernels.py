@@ -110,8 +110,24 @@ def test_other_gathers():
 
 @pytest.mark.parametrize("name", list(RAY))
 def test_ray_design(name):
+    """Sinograms of few rays and small volumes go ray by ray, the rest along detector columns."""
     P = Plan(RAY[name], Options(siddon_bp=SIDDON_BP_RAY))
-    assert back(P) == back(P, 1) == iteration(P)[1] == "bp_column_kernel"
+    assert back(P) == back(P, 1) == "bp_ray_kernel"
+    assert iteration(P)[1] == "bp_column_kernel"
+    P.sensitivity()
+    assert P.last_kernel(PROJECTOR_BACK) == "bp_column_kernel"
+
+
+def test_ray_design_sizes():
+    many = dict(AxPixels=256, TAxPixels=192, AxPixDim=0.375, TAxPixDim=0.375)
+    P = Plan(small_cfg(**many), Options(siddon_bp=SIDDON_BP_RAY))  # 49152 rays a view
+    assert [back(P, n) for n in (1, 4, 5)] == ["bp_ray_kernel", "bp_ray_kernel", "bp_column_kernel"]
+    P = Plan(small_cfg(AxPixels=160, TAxPixels=100, AxPixDim=0.6, TAxPixDim=0.7), Options(siddon_bp=SIDDON_BP_RAY))
+    assert [back(P, n) for n in (10, 11)] == ["bp_ray_kernel", "bp_column_kernel"]  # 16000 rays a view
+    for z, kernel in ((64, "bp_ray_kernel"), (65, "bp_column_kernel")):  # 2^20 voxels, and more
+        P = Plan(small_cfg(Xdim=128, Ydim=128, Zdim=z, XVoxSize=0.25, YVoxSize=0.25, ZVoxSize=0.25),
+                 Options(siddon_bp=SIDDON_BP_RAY))
+        assert back(P, 1) == kernel
 
 
 def test_ray_walk():
