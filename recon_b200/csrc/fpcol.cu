@@ -1321,7 +1321,14 @@ static recon_status_t launch_column(Plan& P, const float* vol, unsigned first, u
     // 16 rounds of them, or a block is one warp (an SM holds 32 blocks).  Wide against not:
     // 256^3 one view 104 against 156 us, 64 views 661 / 686, 360 views 3100 / 2960;
     // 200 x 200 x 120, 32 views 133 / 180, 240 views 681 / 660; 64^3, 90 views 35 / 42.
-    const bool wide = P.col_rows == 32 || (double)grid.x * grid.y * grid.z * (P.col_rows / 32) <= 16.0 * 32.0 * P.sm_count;
+    // Half as many where an unmirrored block is two warps or paths are short, fewer still in
+    // proportion below 128 voxels of x + y: 200 x 200 x 30 unmirrored, 90 and 120 views (11 and
+    // 15 rounds) 314 / 311, 410 / 399 (128^3 mirrored, 180 views, 256 / 263); 64^3 / 400^2, 32
+    // and 48 views (7 and 11) 107 / 110, 150 / 146; 32^3 / 300^2, 24 views (8) 91 / 88.
+    const bool full = (P.col_rows == 128 || P.z_mirror) && E.X + E.Y >= 192;
+    const double rounds = full ? 16.0 : 8.0 * std::min(1.0, (E.X + E.Y) / 128.0);
+    const bool wide =
+        P.col_rows == 32 || (double)grid.x * grid.y * grid.z * (P.col_rows / 32) <= rounds * 32.0 * P.sm_count;
     auto kernel = column_kernel<MODE, LAYOUT, GT, OT>(P, wide);
     note_kernel(RECON_PROJECTOR_FORWARD, wide && P.opt.sum == RECON_SUM_KAHAN && MODE < 3 ? "fp_column_wide_kernel" : "fp_column_kernel");
     if (smem > 48 * 1024) RB_CHECK(allow_dynamic_smem(kernel, kPathSmem));
