@@ -119,8 +119,8 @@ typedef enum { RECON_VOXEL_REFERENCE = 0, RECON_VOXEL_GEOMETRIC = 1 } recon_voxe
  *     of adjacent detector rows cross a column at least one voxel apart.
  *   RAY    -- each ray adds its lengths times its value into 64-bit fixed-point
  *     accumulators (exact, order-independent sums): along detector columns where
- *     the forward projector walks them, else ray by ray through L2-resident
- *     z-slabs.
+ *     the forward projector walks them, else (and for sinograms of few rays into
+ *     small volumes) ray by ray through L2-resident z-slabs.
  *   AUTO   -- GATHER where the rays of adjacent rows cross a voxel column 1 to
  *     1.4 voxels apart (at the depth nearest the source), a ray's piece of one
  *     column spans less than a voxel of z, the volume is at least 128 voxels
