@@ -42,27 +42,36 @@ struct GiveUpPage {
     unsigned* words;
     std::vector<bool> taken;
 };
-std::mutex g_give_up_mutex;
-std::vector<GiveUpPage> g_give_up_pages;
+struct GiveUpPages {
+    std::mutex mutex;
+    std::vector<GiveUpPage> pages;
+};
+// never destroyed: a program's static plan may be destroyed after this library's statics
+GiveUpPages& give_up_pages()
+{
+    static GiveUpPages* const p = new GiveUpPages;
+    return *p;
+}
 }  // namespace
 
 static recon_status_t take_give_up_word(Plan& P)
 {
-    std::lock_guard<std::mutex> lock(g_give_up_mutex);
+    auto& all = give_up_pages();
+    std::lock_guard<std::mutex> lock(all.mutex);
     size_t n = 0, w = kGiveUpWords;
-    for (; n < g_give_up_pages.size(); ++n) {
-        const auto& t = g_give_up_pages[n].taken;
+    for (; n < all.pages.size(); ++n) {
+        const auto& t = all.pages[n].taken;
         w = (size_t)(std::find(t.begin(), t.end(), false) - t.begin());
         if (w < kGiveUpWords) break;
     }
-    if (n == g_give_up_pages.size()) {
+    if (n == all.pages.size()) {
         void* p = nullptr;
         if (posix_memalign(&p, 4096, kGiveUpWords * sizeof(unsigned)) != 0)
             return fail(RECON_ERR_OUT_OF_MEMORY, "no host memory");
-        g_give_up_pages.push_back({static_cast<unsigned*>(p), std::vector<bool>(kGiveUpWords, false)});
+        all.pages.push_back({static_cast<unsigned*>(p), std::vector<bool>(kGiveUpWords, false)});
         w = 0;
     }
-    GiveUpPage& page = g_give_up_pages[n];
+    GiveUpPage& page = all.pages[n];
     unsigned* d = nullptr;
     if (cudaHostGetDevicePointer((void**)&d, page.words, 0) != cudaSuccess) {  // new, or the device was reset
         cudaGetLastError();
@@ -78,8 +87,9 @@ static recon_status_t take_give_up_word(Plan& P)
 
 static void release_give_up_word(unsigned* word)
 {
-    std::lock_guard<std::mutex> lock(g_give_up_mutex);
-    for (GiveUpPage& page : g_give_up_pages)
+    auto& all = give_up_pages();
+    std::lock_guard<std::mutex> lock(all.mutex);
+    for (GiveUpPage& page : all.pages)
         if (word >= page.words && word < page.words + kGiveUpWords) page.taken[word - page.words] = false;
 }
 
